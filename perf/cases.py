@@ -320,3 +320,144 @@ def tolerance(case):
         # rotations round twice per element in the storage type, sin and cos may differ by one unit in its last place
         return {"rel": 1e-3 if case["dtype"] == "fp16" else 8e-3, "max": 2e-2 if case["dtype"] == "fp16" else 1e-1}
     return {"rel": 1e-2 if case["dtype"] == "bf16" else 4e-3, "max": 0.9}
+
+
+# ---- the same in 64 bits ---------------------------------------------------------------------------------------------
+EXACT_MAX_PROMPT = 8192      # longer prompts: the [heads, L, L] scores in 64 bits would take too long and too much memory
+
+
+def _select(pooled, k):
+    """Positions of the k largest of the last dimension (the lowest ones of equal scores), ascending."""
+    order = torch.sort(pooled, dim=-1, descending=True, stable=True).indices[..., :k]
+    return torch.sort(order, dim=-1).values
+
+
+def _exact_sequence(case, layers, heads, padded):
+    """Outputs [n, H, D] of every layer for one prompt; layers: q [H, n, D], k / v [G, n, D] in 64 bits."""
+    outs, chosen = [], None
+    n = layers[0][0].shape[1]
+    dense_only = n <= 128 and not padded
+    tiles = -(-n // TILE)
+    budget = max(0, min(max(128, int(case["pct"] / 100 * n)), n) - TILE)
+    rolling = case["rolling"] and n > 128
+    budgets = [min(budget, max(128, int(case["pct"] * t * TILE / 100))) if rolling else budget for t in range(tiles)]
+    for i, (q, k, v) in enumerate(layers):
+        dev = q.device
+        out = torch.zeros(H, n, D, dtype=torch.float64, device=dev)
+        if dense_only or _is_anchor(i):
+            chosen = [] if not dense_only else None
+            causal = torch.ones(n, n, dtype=torch.bool, device=dev).tril()
+            for g in range(G):
+                s = (q[g * 4:g * 4 + 4] @ k[g].T) * SCALE
+                p = torch.softmax(s.masked_fill(~causal, -math.inf), dim=-1)
+                del s
+                if dense_only or i == 0:
+                    out[g * 4:g * 4 + 4] = p @ v[g]
+                if not dense_only:
+                    chosen.append([_select(p[:, t * TILE:(t + 1) * TILE, :t * TILE].sum((0, 1)), min(budgets[t], t * TILE))
+                                   for t in range(tiles)])
+                del p
+        if not dense_only and i > 0:
+            for g in range(G):
+                rows = chosen[g if _is_anchor(i) else heads[i][g]]
+                for t in range(tiles):
+                    a, e = t * TILE, min((t + 1) * TILE, n)
+                    keys = torch.cat([rows[t], torch.arange(a, e, device=dev)])
+                    s = (q[g * 4:g * 4 + 4, a:e] @ k[g, keys].T) * SCALE
+                    later = keys[None, :] > torch.arange(a, e, device=dev)[:, None]
+                    out[g * 4:g * 4 + 4, a:e] = torch.softmax(s.masked_fill(later, -math.inf), dim=-1) @ v[g, keys]
+        outs.append(out.transpose(0, 1))
+    return outs
+
+
+def _exact_prefill(case, state):
+    if case["length"] > EXACT_MAX_PROMPT:
+        return None
+    L, lens = case["length"], _lengths(case)
+    heads = _head_mapping(case["layers"])
+    outs = [torch.zeros(case["batch"], L, H, D, dtype=torch.float64, device=state["layers"][0][1].device)
+            for _ in range(case["layers"])]
+    padded = any(n != L for n in lens)                       # a batch in which nothing is padded runs as any other
+    for b, n in enumerate(lens):
+        layers = [[x[b, :, L - n:].double() for x in (q, k, v)] for _, q, k, v in state["layers"]]
+        for out, one in zip(outs, _exact_sequence(case, layers, heads, padded)):
+            out[b, L - n:] = one
+    return outs
+
+
+def _exact_token(case, layers, n, longest):
+    """Outputs [H, D] of every layer for one new token over n cached ones; layers: q [H, D], k / v [G, n, D]."""
+    outs, chosen = [], None
+    heads = _head_mapping(case["layers"])
+    budget = n if n <= 128 else min(max(128, int(case["pct"] / 100 * n)), n) - TILE
+    for i, (q, kv) in enumerate(layers):
+        k, v = kv()
+        q = q.view(G, 4, D)
+        if longest <= 128 or _is_anchor(i):
+            p = torch.softmax((q @ k.transpose(1, 2)) * SCALE, dim=-1)
+            chosen = _select(p.sum(1), budget) if longest > 128 else None
+        if longest <= 128 or i == 0:
+            out = p @ v
+        else:
+            rows = chosen if _is_anchor(i) else chosen[heads[i]]
+            rows = rows[:, :, None].expand(-1, -1, D)
+            out = torch.softmax((q @ k.gather(1, rows).transpose(1, 2)) * SCALE, dim=-1) @ v.gather(1, rows)
+        outs.append(out.reshape(H, D))
+    return outs
+
+
+def _exact_hf_decode(case, state):
+    L, per_sequence = case["context"], []
+    lens = _lengths(case)
+    for b, n in enumerate(lens):
+        layers = [(q[b, :, 0].double(), lambda k=k, v=v: (k[b, :, L - n:].double(), v[b, :, L - n:].double()))
+                  for _, q, k, v in state["layers"]]
+        per_sequence.append(_exact_token(case, layers, n, max(lens)))
+    return [torch.stack(rows).unsqueeze(1) for rows in zip(*per_sequence)]
+
+
+def _exact_paged_decode(case, state):
+    per_sequence = []
+    lens = _lengths(case)
+    for b, n in enumerate(lens):
+        pages = state["table"][b, :-(-n // PAGE)].long()
+
+        def rows(cache, scale):
+            x = cache[pages].double()
+            if scale is not None:
+                x = x * scale[pages].double()[:, None, :, None]
+            return x.reshape(-1, G, D)[:n].transpose(0, 1)
+
+        layers = [(q[b].double(), lambda c=state["caches"][i & 1]: (rows(c[0], c[2]), rows(c[1], c[3])))
+                  for i, q in enumerate(state["queries"])]
+        per_sequence.append(_exact_token(case, layers, n, max(lens)))
+    return [torch.stack(rows) for rows in zip(*per_sequence)]
+
+
+def _exact_append(case, state):
+    B, T, start = case["batch"], case["tokens"], case["start"]
+    pos = start + torch.arange(T, device=state["q"].device)
+    angle = pos.double()[:, None] * state["inv_freq"].double()
+    cos, sin = (f(torch.cat([angle, angle], -1))[None, :, None] for f in (torch.cos, torch.sin))
+
+    def turned(x, gain):
+        x = x.double()
+        if gain is not None:
+            x = x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + 1e-6) * gain.double()
+        return x * cos + torch.cat([-x[..., D // 2:], x[..., :D // 2]], -1) * sin
+
+    page, slot = state["table"].long()[:, pos // PAGE], (pos % PAGE).expand(B, T)
+    caches = []
+    for cache, new in ((state["k_cache"], turned(state["k"], state["gains"][1])), (state["v_cache"], state["v"].double())):
+        cache = cache.double()
+        cache[page, slot] = new
+        caches.append(cache)
+    return turned(state["q"], state["gains"][0]), caches[0], caches[1]
+
+
+def exact(case, seed):
+    """What `run` returns for these inputs, in 64 bits and without the library's kernels; None for a case that would take
+    too long.  Keys whose scores differ by less than the library's rounding may be selected differently."""
+    state = prepare(case, seed)
+    return {"prefill": _exact_prefill, "hf_decode": _exact_hf_decode, "paged_decode": _exact_paged_decode,
+            "append": _exact_append}[case["kind"]](case, state)
