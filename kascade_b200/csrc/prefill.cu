@@ -25,15 +25,15 @@
 //   with V, sparse (512 threads): warps 8-10 gather the selected K rows and warps 11, 14, 15 the V rows
 //     with cp.async (16-byte chunks, 16 lanes per 256-byte row, written directly in the
 //     128-byte-swizzled operand layout of umma.cuh); warp 12 issues Q.K^T, warp 13 P.V.
-//   without V (512 threads):      warps 0-11 three softmax / reducer warpgroups (key blocks j = w mod 3);
-//     warp 12 lane 0 TMA copies, warp 13 issues Q.K^T.
+//   without V (640 threads):      warps 0-15 four softmax / reducer warpgroups (key block n of the CTA belongs
+//     to warpgroup n mod 4); warp 16 lane 0 TMA copies, warp 17 issues Q.K^T.
 // setmaxnreg moves registers from the producer / MMA warpgroups to the softmax warpgroups.
 // Hand-offs are mbarriers; every wait is bounded (umma::mbar_wait) and a kernel that gives up
 // records a code in the device status word, drains its copies, frees its tensor memory and returns.
 //
 // Tensor memory (512 columns).  With V: S0 [0,128), S1 [128,256), P0 [256,320), P1 [320,384) (fp16 pairs,
 // the A operand of P.V), O [384,512) - one accumulator for both streams, see the softmax role.
-// Without V: S0, S1, S2.
+// Without V: S0, S1, S2, S3.
 #include <cuda.h>
 #include <stdlib.h>
 
@@ -51,7 +51,7 @@ namespace kb200 {
 enum PrefillMode { kDenseAttn = 0, kDenseLse = 1, kSparse = 2, kPool = 3 };
 
 constexpr int kStageBytes = 128 * kD * 2;     // one 128-row operand tile (32 KB)
-constexpr int kNKMax = 6;                     // K ring: 3 stages with a V ring, 6 without
+constexpr int kNKMax = 4;                     // K ring: 3 stages with a V ring, 4 without
 constexpr int kNV = 3;
 constexpr float kRescaleLog2 = 8.0f;          // see the softmax role
 constexpr int kPadAllowance = 512;            // tiles need 1024-byte alignment
@@ -100,37 +100,6 @@ __device__ __forceinline__ void cp_arrive_noinc(uint64_t* bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(umma::smem_addr(bar)) : "memory");
 }
 __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
-// 2^x on the FMA pipes, for x <= 127: the special-function unit delivers 16 results per clock and SM,
-// which is what bounds the softmax; every fourth exponential goes this way instead.  x is rounded
-// to the nearest integer n by adding 1.5 * 2^23 (n lands in the low mantissa bits), 2^(x - n) on
-// [-0.5, 0.5] is a degree-4 polynomial (relative error 3e-6), and n is added to the exponent field.
-// Share of the exponentials of the lse and pool passes that goes to the FMA pipes: every fourth one, and with
-// EXTRA = n > 0 one more in every n-th group of four.  Measured at 32 768 tokens: the lse pass is fastest with
-// a quarter (3/8: +11 %), the pool pass, whose other arithmetic is packed two per instruction, with 3/8 (-4 %).
-#ifndef KB200_POLY_EXTRA_LSE
-#define KB200_POLY_EXTRA_LSE 0
-#endif
-#ifndef KB200_POLY_EXTRA_POOL
-#define KB200_POLY_EXTRA_POOL 2
-#endif
-template <int EXTRA>
-__device__ __forceinline__ constexpr bool poly_also(int i) {
-  return EXTRA > 0 && ((i >> 2) % (EXTRA > 0 ? EXTRA : 1)) == 0;
-}
-__device__ __forceinline__ float ex2_fma(float x) {
-#ifdef KB200_NO_FMA_EXP
-  return ex2(x);
-#endif
-  x = fmaxf(x, -120.0f);                               // also maps -inf (masked) to 2^-120 ~ 0
-  const float t = x + 12582912.0f;
-  const float f = x - (t - 12582912.0f);
-  float q = 0.009585312567651272f;
-  q = fmaf(q, f, 0.05590597912669182f);
-  q = fmaf(q, f, 0.24024048447608948f);
-  q = fmaf(q, f, 0.6931242942810059f);
-  q = fmaf(q, f, 1.0f);
-  return __uint_as_float(__float_as_uint(q) + (__float_as_uint(t) << 23));
-}
 // Two fp32 operations per instruction (sm_100: fma / add on register pairs) and the three-input maximum:
 // the softmax warps are bound by the number of instructions they issue, not by a single pipe, so every
 // per-element instruction that two elements can share is worth taking.  Results are those of the scalar
@@ -158,6 +127,39 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
   asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
+// 2^x of a register pair on the FMA pipes, for x <= 127: the special-function unit delivers 16 results per clock
+// and SM, which alone would hold a 128 x 128 block for 1024 cycles, so the passes that only sum their exponentials
+// (lse, pool) take a share of them this way.  x is rounded to the nearest integer n by adding 1.5 * 2^23 (n lands in
+// the low mantissa bits), 2^(x - n) on [-0.5, 0.5] is a degree-4 polynomial (relative error 3e-6), and n is added to
+// the exponent field.  Everything but the clamp and the exponent is two-element instructions.
+__device__ __forceinline__ uint64_t ex2_fma2(uint64_t x2) {
+  float x0, x1;
+  unpair_f(x2, x0, x1);
+  const uint64_t x = pair_f(fmaxf(x0, -120.0f), fmaxf(x1, -120.0f));   // also maps -inf (masked) to 2^-120 ~ 0
+  const uint64_t t = add2(x, pair_f(12582912.0f, 12582912.0f));
+  const uint64_t n = add2(t, pair_f(-12582912.0f, -12582912.0f));
+  const uint64_t f = fma2(n, pair_f(-1.0f, -1.0f), x);
+  uint64_t q = pair_f(0.009585312567651272f, 0.009585312567651272f);
+  q = fma2(q, f, pair_f(0.05590597912669182f, 0.05590597912669182f));
+  q = fma2(q, f, pair_f(0.24024048447608948f, 0.24024048447608948f));
+  q = fma2(q, f, pair_f(0.6931242942810059f, 0.6931242942810059f));
+  q = fma2(q, f, pair_f(1.0f, 1.0f));
+  float q0, q1, t0, t1;
+  unpair_f(q, q0, q1);
+  unpair_f(t, t0, t1);
+  return pair_u(__float_as_uint(q0) + (__float_as_uint(t0) << 23), __float_as_uint(q1) + (__float_as_uint(t1) << 23));
+}
+// 2^x of pair number `pair` (0..15) of 32 values: kPolyShare of the 16 pairs, evenly spread, go to the FMA pipes.  The
+// two-element fma occupies the heavy FMA pipe for two cycles, so that pipe (256 + 56 * share cycles per block) and
+// the special-function unit (1024 - 64 * share) meet at a share of 5-6.  Measured with four streams at 8192 tokens,
+// share 0 / 3 / 4 / 5 / 6 / 16: pool 364 / 313 / 301 / 292 / 295 / 481 us, lse 361 / 325 / 326 / 331 / 333 / 494 us.
+constexpr int kPolyShare = 5;
+__device__ __forceinline__ uint64_t ex2_pair(int pair, uint64_t x) {
+  if (((pair + 1) * kPolyShare >> 4) != (pair * kPolyShare >> 4)) return ex2_fma2(x);
+  float x0, x1;
+  unpair_f(x, x0, x1);
+  return pair_f(ex2(x0), ex2(x1));
+}
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;\n" : "=f"(d) : "f"(a), "f"(b), "f"(c));
@@ -184,21 +186,19 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 // Barriers and small exchange buffers; lives in dynamic shared memory behind the operand tiles so that
 // the 7 x 32 KB tiles, the alignment padding and this block together stay inside the 227 KB limit.
 struct PfShared {
-  uint64_t bar_q, bar_qempty, bar_kfull[kNKMax], bar_kempty[kNKMax], bar_vfull[kNV], bar_vempty[kNV];
-  uint64_t bar_sfull[3], bar_pready[3], bar_odone[3], bar_x, bar_ofree, bar_lse[3], bar_sfree[2], bar_turn[2];
+  uint64_t bar_q[2], bar_qempty[2], bar_kfull[kNKMax], bar_kempty[kNKMax], bar_vfull[kNV], bar_vempty[kNV];
+  uint64_t bar_sfull[4], bar_pready[4], bar_odone[2], bar_x, bar_ofree, bar_lse[4], bar_sfree[2];
   uint32_t tmem;
   int give_up;
   int abort;                                           // copy of the device status word taken at CTA start
-  union {
-    float xchg[2][2][128];                             // softmax modes: [m (with V: row reference) | l][warpgroup][row]
-    float lse[2][2][128];                              // pool mode: lse2 of the tile's rows [warpgroup][tile parity]
-  };
+  float xchg[2][2][128];                               // modes with V: [row reference | l][warpgroup][row]
 };
 static_assert(sizeof(PfShared) <= 2560, "PfShared grew");
 constexpr int kSmemAttn = kStageBytes * (1 + 3 + kNV) + kPadAllowance + 2560;   // = 232448, the sm_100 limit
-constexpr int kNKNoV = 5;                     // K ring of the modes without V
-constexpr int kXchgNoV = 3 * 2 * 128 * 4;     // their exchange area behind PfShared: three streams x two values x 128 rows
-constexpr int kSmemNoV = kStageBytes * (1 + kNKNoV) + kPadAllowance + 2560 + kXchgNoV;
+constexpr int kNQNoV = 2, kNKNoV = 4;         // Q tiles and K ring of the modes without V
+constexpr int kStreamsNoV = 4;
+constexpr int kXchgNoV = kStreamsNoV * 2 * 128 * 4;   // their exchange area behind PfShared: two values per stream and row
+constexpr int kSmemNoV = kStageBytes * (kNQNoV + kNKNoV) + kPadAllowance + 2560 + kXchgNoV;
 
 // One work item = one query tile of one KV head of one sequence.
 struct TileItem {
@@ -251,18 +251,18 @@ struct PfCfg {
   static constexpr bool kHasV = MODE == kDenseAttn || MODE == kSparse;
   static constexpr bool kIsPool = MODE == kPool;
   static constexpr bool kGather = MODE == kSparse;
-  // softmax warpgroups (streams): two with V; three without V, where nothing but latency limits them
-  static constexpr int kStreams = kHasV ? 2 : 3;
+  // softmax warpgroups (streams): two with V; four without, where a block has no accumulator and no probabilities
+  // to keep and a thread holds half a row at a time (104 registers).  Against three streams that hold whole rows, at
+  // 16384 tokens: lse 1405 -> 1285 us, pool 1345 -> 1190 us, together with the issuer's early look and the second Q tile.
+  static constexpr int kStreams = kHasV ? 2 : kStreamsNoV;
   static constexpr int kSoftmaxWarps = 4 * kStreams;
-  // warps that issue Q.K^T without V: two taking the key blocks in turn paid off in the pool mode (-4 %),
-  // not in the lse mode
-  static constexpr int kIssuers = kIsPool ? 2 : 1;
-  static constexpr int kThreads = (kGather || !kHasV) ? 512 : 384;
+  static constexpr int kThreads = !kHasV ? 640 : kGather ? 512 : 384;
+  static constexpr int kNQ = kHasV ? 1 : kNQNoV;
   static constexpr int kNK = kHasV ? 3 : kNKNoV;
   static constexpr int kProducerArrivals = 1;                   // Q tile: one thread announces the TMA bytes
   static constexpr int kRingArrivals = kGather ? 96 : 1;        // K / V stage: three gather warps each
-  static constexpr int kProducerWarp0 = kHasV ? 8 : 12;
-  static constexpr int kMmaWarp = kGather ? 12 : (kHasV ? 9 : 13);
+  static constexpr int kProducerWarp0 = kHasV ? 8 : 16;
+  static constexpr int kMmaWarp = kGather ? 12 : (kHasV ? 9 : 17);
 };
 
 template <int MODE, bool BF16>
@@ -285,15 +285,16 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
     return;
   }
   uint8_t* smem = smem_raw + pad;
-  constexpr int kTiles = 1 + kNK + (HAS_V ? kNV : 0);
+  constexpr int kNQ = Cfg::kNQ;
+  constexpr int kTiles = kNQ + kNK + (HAS_V ? kNV : 0);
   PfShared& sh = *reinterpret_cast<PfShared*>(smem + kTiles * kStageBytes);
   // an earlier CTA or kernel gave up a bounded wait: do not queue up more waits behind it.  One thread
   // reads the word and the whole CTA takes the same decision.
   if (tid == 0) sh.abort = *reinterpret_cast<volatile int*>(&g_status_word);
   __syncthreads();
   if (sh.abort != 0) return;
-  // modes without V: [3 streams][2][128] floats behind PfShared (partial row statistics / staged lse values)
-  float* const xchg3 = reinterpret_cast<float*>(smem + kTiles * kStageBytes + 2560);
+  // modes without V: [4 streams][2][128] floats behind PfShared (partial row statistics / staged lse values)
+  float* const xchg_nov = reinterpret_cast<float*>(smem + kTiles * kStageBytes + 2560);
   uint64_t* bar_kfull = sh.bar_kfull;
   uint64_t* bar_kempty = sh.bar_kempty;
   uint64_t* bar_vfull = sh.bar_vfull;
@@ -303,23 +304,20 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
   uint64_t* bar_odone = sh.bar_odone;
   int& give_up = sh.give_up;
   const uint32_t q_s = smem_addr(smem);
-  const uint32_t k_s = q_s + kStageBytes;
+  const uint32_t k_s = q_s + kNQ * kStageBytes;
   const uint32_t v_s = k_s + kNK * kStageBytes;
 
   if (tid == 0) {
-    mbar_init(&sh.bar_q, Cfg::kProducerArrivals);
-    mbar_init(&sh.bar_qempty, HAS_V ? 1 : Cfg::kIssuers);   // one arrival per Q.K^T issuer
-    mbar_init(&sh.bar_turn[0], 1);
-    mbar_init(&sh.bar_turn[1], 1);
+    for (int i = 0; i < 2; ++i) { mbar_init(&sh.bar_q[i], Cfg::kProducerArrivals); mbar_init(&sh.bar_qempty[i], 1); }
     for (int i = 0; i < kNK; ++i) { mbar_init(&bar_kfull[i], HAS_V ? Cfg::kRingArrivals : Cfg::kProducerArrivals); mbar_init(&bar_kempty[i], 1); }
     for (int i = 0; i < kNV; ++i) { mbar_init(&bar_vfull[i], Cfg::kRingArrivals); mbar_init(&bar_vempty[i], 1); }
     // each softmax warpgroup (128 threads) owns every other key block of a tile
-    for (int i = 0; i < 3; ++i) {
+    for (int i = 0; i < 4; ++i) {
       mbar_init(&bar_sfull[i], 1);
       mbar_init(&bar_pready[i], 128);
-      mbar_init(&bar_odone[i], 1);
+      mbar_init(&sh.bar_lse[i], 128);
     }
-    for (int i = 0; i < 3; ++i) mbar_init(&sh.bar_lse[i], 128);
+    for (int i = 0; i < 2; ++i) mbar_init(&bar_odone[i], 1);
     for (int i = 0; i < 2; ++i) mbar_init(&sh.bar_sfree[i], 128);
     mbar_init(&sh.bar_x, Cfg::kSoftmaxWarps * 32);
     mbar_init(&sh.bar_ofree, Cfg::kSoftmaxWarps * 32);
@@ -457,11 +455,14 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
       if (item >= n_items) continue;
       const TileItem it = decode_item<MODE>(p, item);
       if (it.nb == 0) continue;
-      ok = mbar_wait(&sh.bar_qempty, (qn & 1) ^ 1, &give_up, 13);
+      // with two Q tiles (modes without V) the next one is on its way while the current one's products run
+      const int qb = qn % kNQ;
+      ok = mbar_wait(&sh.bar_qempty[qb], ((qn / kNQ) & 1) ^ 1, &give_up, 13);
       if (!ok) break;
-      mbar_arrive_expect_tx(&sh.bar_q, kStageBytes);
-      tma_load_4d(q_s, &tm_q, 0, it.g * kHg, it.row0 + it.tile_start, it.b, &sh.bar_q);
-      tma_load_4d(q_s + kStageBytes / 2, &tm_q, 64, it.g * kHg, it.row0 + it.tile_start, it.b, &sh.bar_q);
+      const uint32_t q_dst = q_s + qb * kStageBytes;
+      mbar_arrive_expect_tx(&sh.bar_q[qb], kStageBytes);
+      tma_load_4d(q_dst, &tm_q, 0, it.g * kHg, it.row0 + it.tile_start, it.b, &sh.bar_q[qb]);
+      tma_load_4d(q_dst + kStageBytes / 2, &tm_q, 64, it.g * kHg, it.row0 + it.tile_start, it.b, &sh.bar_q[qb]);
       ++qn;
       for (int j = 0; j < it.nb; ++j) {
         ok = mbar_wait(&bar_kempty[st], ph, &give_up, 11);
@@ -497,79 +498,62 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
   };
 
   // ================================ MMA issuer, modes without V ===================================
-  // One warp issues, or (Cfg::kIssuers == 2) two, taking the key blocks in turn (global block count
-  // even / odd): an issuing lane is
-  // held up while the tensor core works through its queue, so with one issuer the barrier waits of
-  // block n+1 would start only after block n has run; with two, one warp waits while the other's
-  // products execute.  Both walk the same block sequence and keep the same counters.  A wait names a
-  // barrier phase only by its parity, so an issuer must never wait on a barrier that is still two
-  // phases back: the issuer of block n passes a token to the other one as soon as its own "S buffer
-  // free" wait is over, and the other one starts its waits for block n+1 only then.
-  auto mma_role = [&](const int me) {
+  // The key blocks of a CTA are numbered n = 0, 1, 2, ... across all its tiles; block n goes through S buffer
+  // n % kStreams and K stage n % kNK.  The tensor core holds only a few products in its queue, so an issuer that
+  // starts its waits for block n + 1 after block n's products leaves it idle between blocks: it looks at block
+  // n + 1's barriers before the last product of block n, and waits only if they were not complete by then.  With
+  // the softmax work left out, this and the second Q tile took the pass from 254 to 191 us at 8192 tokens (the
+  // products alone: 123 us).  The look must not wait itself: with try_wait, which may suspend the warp, it cost time.
+  auto mma_role = [&]() {
     constexpr uint32_t idesc_qk = idesc_f16(128, 128, 0, 0, BF16);
-    constexpr int NS = Cfg::kStreams;                   // S buffers = softmax streams; block j goes to buffer j % NS
-    constexpr int kIssuers = Cfg::kIssuers;
-    int k_st = 0, k_ph = 0, qn = 0, gb = 0, turns = 0;  // K ring, Q tiles, global block count, tokens taken
-    int used[NS];                                      // blocks written into each S buffer so far (by either issuer)
-#pragma unroll
-    for (int i = 0; i < NS; ++i) used[i] = 0;
-    bool ok = true;
+    constexpr int NS = Cfg::kStreams;
+    int n = 0, qn = 0;
+    bool ok = true, have = false;                       // have: block n's barriers have been seen complete
     // the whole warp runs this role with uniform control flow; one elected lane issues
     const bool el = elect_one();
-    const uint32_t q_lo = desc_lo(q_s, 16), k_lo0 = desc_lo(k_s, 16);
+    const uint32_t q_lo0 = desc_lo(q_s, 16), k_lo0 = desc_lo(k_s, 16);
     for (int k = 0; k < n_rounds && ok; ++k) {
       const int item = item_of(k);
       if (item >= n_items) continue;
       const TileItem it = decode_item<MODE>(p, item);
       if (it.nb == 0) continue;
-      ok = mbar_wait(&sh.bar_q, qn & 1, &give_up, 21);
+      const int qb = qn % kNQ;
+      ok = mbar_wait(&sh.bar_q[qb], (qn / kNQ) & 1, &give_up, 21);
       if (!ok) break;
       ++qn;
-      int w = 0;
-      bool issued_here = false;
-      for (int j = 0; j < it.nb && ok; ++j, ++gb) {
-        if (kIssuers == 1 || (gb & 1) == me) {
-          if (kIssuers == 2 && gb > 0) {                 // the other issuer is past its waits for block gb - 1
-            ok = mbar_wait(&sh.bar_turn[me], turns & 1, &give_up, 27);
-            if (!ok) break;
-            ++turns;
-          }
+      const uint32_t q_lo = q_lo0 + qb * (kStageBytes >> 4);
+      for (int j = 0; j < it.nb; ++j) {
+        const int w = n % NS, st = n % kNK;
+        if (!have) {
           // S buffer w may be overwritten once the block issued into it before has been consumed
-#pragma unroll
-          for (int i = 0; i < NS; ++i) {
-            if (i == w && used[i] > 0) ok = mbar_wait(&bar_pready[i], (used[i] - 1) & 1, &give_up, 23);
-          }
+          if (n >= NS) ok = mbar_wait(&bar_pready[w], (n / NS - 1) & 1, &give_up, 23);
+          if (ok) ok = mbar_wait(&bar_kfull[st], (n / kNK) & 1, &give_up, 22);
           if (!ok) break;
-          if (kIssuers == 2 && el) mbar_arrive(&sh.bar_turn[me ^ 1]);
-          ok = mbar_wait(&bar_kfull[k_st], k_ph, &give_up, 22);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t k_lo = k_lo0 + k_st * (kStageBytes >> 4);
-          const uint32_t d = t_s0 + w * 128;
-          if (el) {
-#pragma unroll
-            for (int ks = 0; ks < 8; ++ks) {
-              const uint32_t off = (ks >> 2) * (kStageBytes / 2 / 16) + (ks & 3) * 2;
-              if (POOL) mma_ss_lo(d, k_lo + off, q_lo + off, idesc_qk, ks > 0);     // S^T: lanes = keys
-              else mma_ss_lo(d, q_lo + off, k_lo + off, idesc_qk, ks > 0);          // S: lanes = (query, head) rows
-            }
-            mma_commit(&bar_kempty[k_st]);
-            mma_commit(&bar_sfull[w]);
-          }
-          __syncwarp();
-          issued_here = true;
         }
+        tc_fence_after();
+        const uint32_t k_lo = k_lo0 + st * (kStageBytes >> 4);
+        const uint32_t d = t_s0 + w * 128;
+        auto issue = [&](int ks) {
+          const uint32_t off = (ks >> 2) * (kStageBytes / 2 / 16) + (ks & 3) * 2;
+          if (POOL) mma_ss_lo(d, k_lo + off, q_lo + off, idesc_qk, ks > 0);     // S^T: lanes = keys
+          else mma_ss_lo(d, q_lo + off, k_lo + off, idesc_qk, ks > 0);          // S: lanes = (query, head) rows
+        };
+        if (el) {
 #pragma unroll
-        for (int i = 0; i < NS; ++i) if (i == w) ++used[i];
-        if (++k_st == kNK) { k_st = 0; k_ph ^= 1; }
-        if (++w == NS) w = 0;
+          for (int ks = 0; ks < 7; ++ks) issue(ks);
+        }
+        ++n;
+        have = (n < NS || mbar_test_wait(&bar_pready[n % NS], (n / NS - 1) & 1)) &&
+               mbar_test_wait(&bar_kfull[n % kNK], (n / kNK) & 1);
+        have = __all_sync(0xFFFFFFFFu, have);           // the lanes may have looked at different moments
+        if (el) {
+          issue(7);
+          mma_commit(&bar_kempty[st]);
+          mma_commit(&bar_sfull[w]);
+          if (j + 1 == it.nb) mma_commit(&sh.bar_qempty[qb]);   // the tile's last product is queued
+        }
+        __syncwarp();
       }
-      if (!ok) break;
-      // Q may be replaced once BOTH issuers' products of this tile have completed (two arrivals)
-      if (el) {
-        if (issued_here) mma_commit(&sh.bar_qempty); else mbar_arrive(&sh.bar_qempty);
-      }
-      __syncwarp();
     }
   };
 
@@ -603,12 +587,12 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
         // Sparse mode: this warp also fetches the Q tile (two TMA boxes), as soon as the previous tile's
         // last Q.K^T has completed; the next tile's Q is pulled into L2 meanwhile, so that its copy
         // starts from there.
-        ok = mbar_wait(&sh.bar_qempty, (qn & 1) ^ 1, &give_up, 13);
+        ok = mbar_wait(&sh.bar_qempty[0], (qn & 1) ^ 1, &give_up, 13);
         if (!ok) break;
         if (el) {
-          mbar_arrive_expect_tx(&sh.bar_q, kStageBytes);
-          tma_load_4d(q_s, &tm_q, 0, it.g * kHg, it.row0 + it.tile_start, it.b, &sh.bar_q);
-          tma_load_4d(q_s + kStageBytes / 2, &tm_q, 64, it.g * kHg, it.row0 + it.tile_start, it.b, &sh.bar_q);
+          mbar_arrive_expect_tx(&sh.bar_q[0], kStageBytes);
+          tma_load_4d(q_s, &tm_q, 0, it.g * kHg, it.row0 + it.tile_start, it.b, &sh.bar_q[0]);
+          tma_load_4d(q_s + kStageBytes / 2, &tm_q, 64, it.g * kHg, it.row0 + it.tile_start, it.b, &sh.bar_q[0]);
           if (k + 1 < n_rounds) {
             const int nitem = item_of(k + 1);
             if (nitem < n_items) {
@@ -622,7 +606,7 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
         }
         __syncwarp();
       }
-      ok = mbar_wait(&sh.bar_q, qn & 1, &give_up, 21);
+      ok = mbar_wait(&sh.bar_q[0], qn & 1, &give_up, 21);
       if (!ok) break;
       ++qn;
       for (int j = 0; j < it.nb; ++j) {
@@ -648,7 +632,7 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
           }
           mma_commit(&bar_kempty[k_st]);
           mma_commit(&bar_sfull[w]);
-          if (j + 1 == it.nb) mma_commit(&sh.bar_qempty);  // the tile's last Q.K^T is queued: Q may be replaced
+          if (j + 1 == it.nb) mma_commit(&sh.bar_qempty[0]);  // the tile's last Q.K^T is queued: Q may be replaced
         }
         __syncwarp();
         ++iss;
@@ -974,20 +958,20 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
   };
 
   // ================================ softmax statistics only (no V) ================================
-  // Three warpgroups, three independent streams: warpgroup w owns the key blocks j = w, w+3, ... of
-  // every tile with its own S buffer and its own running (max, sum) per row, so the tcgen05.ld / max /
-  // ex2 phases of one stream overlap those of the others and nothing is exchanged per block (with two
-  // streams no unit was busy more than 64 %: three warps per SM sub-partition hide each other's
-  // latencies better).  The partial results of a row are merged like split-K partials in the epilogue.
+  // Four warpgroups, four independent streams: warpgroup w owns the key blocks n = w mod 4 of the CTA with its own S
+  // buffer and its own running (max, sum) per row, so the tcgen05.ld / max / ex2 phases of one stream overlap
+  // those of the others and nothing is exchanged per block.  A thread reads its row from tensor memory in halves of
+  // 64 values (the lower half twice), which is what lets four streams fit the register file.  The partial results
+  // of a row are merged like split-K partials in the epilogue.
   auto softmax_role = [&]() {
     const int wg = warp >> 2;
     const int row = (warp & 3) * 32 + lane, q_local = row >> 2;
     const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t ts = t_s0 + wg * 128 + lane_sel;   // this stream's S buffer
     constexpr int NS = Cfg::kStreams;
-    float* const xm = xchg3;                           // [NS][128] partial maxima
-    float* const xl = xchg3 + NS * 128;                // [NS][128] partial sums
-    int done_mine = 0, tiles_done = 0;                 // blocks finished by this stream, tiles finished
+    float* const xm = xchg_nov;                           // [NS][128] partial maxima
+    float* const xl = xchg_nov + NS * 128;                // [NS][128] partial sums
+    int n0 = 0, tiles_done = 0;                        // blocks of the tiles before this one, tiles finished
     bool ok = true;
     for (int k = 0; k < n_rounds && ok; ++k) {
       const int item = item_of(k);
@@ -996,62 +980,71 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
       if (it.nb == 0) continue;
       const int tok = it.tile_start + q_local;
       const int off = it.tile_start;                    // slot - off = key position inside the tile
-      const int n_mine = it.nb > wg ? (it.nb - wg + NS - 1) / NS : 0;
       float m_run = -INFINITY, l_run = 0.f;             // m_run in the scaled (log2) domain
-      for (int j = wg, jj = 0; j < it.nb; j += NS, ++jj) {
-        ok = mbar_wait(&bar_sfull[wg], (done_mine + jj) & 1, &give_up, 31);
+      for (int j = (wg + NS - n0 % NS) % NS; j < it.nb; j += NS) {
+        ok = mbar_wait(&bar_sfull[wg], ((n0 + j) / NS) & 1, &give_up, 31);
         if (!ok) break;
         tc_fence_after();
         const int c0 = j * 128 - off;                     // key position (inside the tile) of column 0
         const bool need_mask = (c0 + 127) > 0;            // only the last block(s) of a tile
-        // the whole S row (128 fp32) comes into registers with one round trip to tensor memory
-        uint32_t sr[4][32];
+        uint32_t sa[32], sb[32];
+        auto load_half = [&](int c) {
+          tmem_ld32(ts + c, sa);
+          tmem_ld32(ts + c + 32, sb);
+          tmem_wait_ld();
+          if (need_mask) {
 #pragma unroll
-        for (int part = 0; part < 4; ++part) tmem_ld32(ts + part * 32, sr[part]);
-        tmem_wait_ld();
-        tc_fence_before();
-        mbar_arrive(&bar_pready[wg]);                     // S is in registers: the buffer may be refilled
-        if (need_mask) {
-#pragma unroll
-          for (int part = 0; part < 4; ++part)
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if ((c0 + part * 32 + i) > q_local) sr[part][i] = 0xFF800000u;     // -inf
-        }
+            for (int i = 0; i < 32; ++i) {
+              if ((c0 + c + i) > q_local) sa[i] = 0xFF800000u;     // -inf
+              if ((c0 + c + 32 + i) > q_local) sb[i] = 0xFF800000u;
+            }
+          }
+        };
         float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
-#pragma unroll
-        for (int part = 0; part < 4; ++part) {
+        auto max_half = [&]() {
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
-            mx0 = fmaxf(mx0, __uint_as_float(sr[part][i]));
-            mx1 = fmaxf(mx1, __uint_as_float(sr[part][i + 1]));
-            mx2 = fmaxf(mx2, __uint_as_float(sr[part][i + 2]));
-            mx3 = fmaxf(mx3, __uint_as_float(sr[part][i + 3]));
+            mx0 = max3(mx0, __uint_as_float(sa[i]), __uint_as_float(sa[i + 1]));
+            mx1 = max3(mx1, __uint_as_float(sa[i + 2]), __uint_as_float(sa[i + 3]));
+            mx2 = max3(mx2, __uint_as_float(sb[i]), __uint_as_float(sb[i + 1]));
+            mx3 = max3(mx3, __uint_as_float(sb[i + 2]), __uint_as_float(sb[i + 3]));
           }
-        }
+        };
+        load_half(0);
+        max_half();
+        load_half(64);
+        max_half();
         const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * p.scale2;
         // The reference point of the exponentials only moves when the row maximum has grown by more
         // than 2^kRescaleLog2 (the terms then stay below 2^kRescaleLog2, exact in fp32);
         // lse2 = m + log2(l) holds for any reference point m.
         const float m_new = (mx > m_run + kRescaleLog2) ? mx : m_run;
         const float alpha = ex2(m_run - m_new);
-        float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-#pragma unroll
-        for (int part = 0; part < 4; ++part)
+        uint64_t s01 = 0ull, s23 = 0ull;                    // four partial row sums, two per register pair
+        const uint64_t scale_2 = pair_f(p.scale2, p.scale2), nref_2 = pair_f(-m_new, -m_new);
+        auto sum_part = [&](const uint32_t (&sr)[32]) {
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
-            s0 += ex2(fmaf(__uint_as_float(sr[part][i]), p.scale2, -m_new));
-            s1 += poly_also<KB200_POLY_EXTRA_LSE>(i) ? ex2_fma(fmaf(__uint_as_float(sr[part][i + 1]), p.scale2, -m_new))
-                               : ex2(fmaf(__uint_as_float(sr[part][i + 1]), p.scale2, -m_new));
-            s2 += ex2(fmaf(__uint_as_float(sr[part][i + 2]), p.scale2, -m_new));
-            s3 += ex2_fma(fmaf(__uint_as_float(sr[part][i + 3]), p.scale2, -m_new));
+            s01 = add2(s01, ex2_pair(i >> 1, fma2(pair_u(sr[i], sr[i + 1]), scale_2, nref_2)));
+            s23 = add2(s23, ex2_pair((i >> 1) + 1, fma2(pair_u(sr[i + 2], sr[i + 3]), scale_2, nref_2)));
           }
+        };
+        sum_part(sa);
+        sum_part(sb);
+        load_half(0);
+        tc_fence_before();
+        mbar_arrive(&bar_pready[wg]);                     // S has been read for the last time: the buffer may be refilled
+        sum_part(sa);
+        sum_part(sb);
+        float s0, s1, s2, s3;
+        unpair_f(s01, s0, s1);
+        unpair_f(s23, s2, s3);
         l_run = l_run * alpha + ((s0 + s1) + (s2 + s3));
         m_run = m_new;
       }
       if (!ok) break;
-      done_mine += n_mine;
-      // ---- epilogue: merge the two streams, store ------------------------------------------------
+      n0 += it.nb;
+      // ---- epilogue: merge the streams, store ------------------------------------------------
       // the exchange buffer is free once both warpgroups have finished the previous tile's epilogue
       if (tiles_done > 0) {
         ok = mbar_wait(&sh.bar_ofree, (tiles_done - 1) & 1, &give_up, 37);
@@ -1081,14 +1074,14 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
   };
 
   // ================================ pooled-score reducer =========================================
-  // warpgroup w owns the key blocks j = w, w+3, ... of every tile; thread = key lane, sums over the
+  // warpgroup w owns the key blocks n = w mod 4 of the CTA; thread = key lane, sums over the
   // tile's 128 (query, head) rows, i.e. over the 128 columns of S^T
   auto pool_role = [&]() {
     const int wg = warp >> 2;
     const int key_lane = (warp & 3) * 32 + lane;
     const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t ts = t_s0 + wg * 128 + lane_sel;
-    int done_mine = 0, tiles_seen = 0;
+    int n0 = 0, tiles_seen = 0;                          // blocks and tiles before this one
     bool ok = true;
     for (int k = 0; k < n_rounds && ok; ++k) {
       const int item = item_of(k);
@@ -1096,11 +1089,10 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
       const TileItem it = decode_item<MODE>(p, item);
       if (it.nb == 0) continue;
       constexpr int NS = Cfg::kStreams;
-      const int n_mine = it.nb > wg ? (it.nb - wg + NS - 1) / NS : 0;
       // this warpgroup's copy of the tile's 128 lse2 values (row = 4 * query + head), double-buffered
       // by tile parity: a thread that runs ahead must not overwrite values that a slower thread of
       // the warpgroup still reads for the previous tile
-      float* lse_s = xchg3 + (wg * 2 + (tiles_seen & 1)) * 128;
+      float* lse_s = xchg_nov + (wg * 2 + (tiles_seen & 1)) * 128;
       {
         const int tok = it.tile_start + (key_lane >> 2);
         lse_s[key_lane] =
@@ -1111,37 +1103,42 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
         ++tiles_seen;
       }
       float* prow = p.pooled + (((int64_t)it.b * p.G + it.g) * p.T + it.t) * p.pooled_stride;
-      for (int j = wg, jj = 0; j < it.nb; j += NS, ++jj) {
-        ok = mbar_wait(&bar_sfull[wg], (done_mine + jj) & 1, &give_up, 41);
+      for (int j = (wg + NS - n0 % NS) % NS; j < it.nb; j += NS) {
+        ok = mbar_wait(&bar_sfull[wg], ((n0 + j) / NS) & 1, &give_up, 41);
         if (!ok) break;
         tc_fence_after();
         uint64_t a01 = 0ull, a23 = 0ull;                    // four partial sums, two per register pair
         const uint64_t scale_2 = pair_f(p.scale2, p.scale2);
-        uint32_t sr[4][32];
-#pragma unroll
-        for (int part = 0; part < 4; ++part) tmem_ld32(ts + part * 32, sr[part]);
-        tmem_wait_ld();
-        tc_fence_before();
-        mbar_arrive(&bar_pready[wg]);                      // S^T block is in registers: the buffer is free
-#pragma unroll
-        for (int part = 0; part < 4; ++part)
+        auto sum_part = [&](const uint32_t (&sr)[32], int part) {
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
             // the four rows' lse2 with one 16-byte shared-memory load (the same address for the whole warp)
             const float4 l4 = reinterpret_cast<const float4*>(lse_s)[part * 8 + (i >> 2)];   // holds -lse2
-            float x0, x1, x2, x3;
-            unpair_f(fma2(pair_u(sr[part][i], sr[part][i + 1]), scale_2, pair_f(l4.x, l4.y)), x0, x1);
-            unpair_f(fma2(pair_u(sr[part][i + 2], sr[part][i + 3]), scale_2, pair_f(l4.z, l4.w)), x2, x3);
-            a01 = add2(a01, pair_f(ex2(x0), poly_also<KB200_POLY_EXTRA_POOL>(i) ? ex2_fma(x1) : ex2(x1)));
-            a23 = add2(a23, pair_f(ex2(x2), ex2_fma(x3)));
+            a01 = add2(a01, ex2_pair(i >> 1, fma2(pair_u(sr[i], sr[i + 1]), scale_2, pair_f(l4.x, l4.y))));
+            a23 = add2(a23, ex2_pair((i >> 1) + 1, fma2(pair_u(sr[i + 2], sr[i + 3]), scale_2, pair_f(l4.z, l4.w))));
           }
+        };
+        uint32_t sa[32], sb[32];                            // 64 of the 128 values at a time, the next part on its way
+        tmem_ld32(ts, sa);
+        tmem_wait_ld();
+        tmem_ld32(ts + 32, sb);
+        sum_part(sa, 0);
+        tmem_wait_ld();
+        tmem_ld32(ts + 64, sa);
+        sum_part(sb, 1);
+        tmem_ld32(ts + 96, sb);
+        tmem_wait_ld();
+        tc_fence_before();
+        mbar_arrive(&bar_pready[wg]);                      // the S^T block has been read: the buffer is free
+        sum_part(sa, 2);
+        sum_part(sb, 3);
         float a0, a1, a2, a3;
         unpair_f(a01, a0, a1);
         unpair_f(a23, a2, a3);
         const int key = j * 128 + key_lane;
         if (key < it.tile_start) prow[key] = (a0 + a1) + (a2 + a3);
       }
-      done_mine += n_mine;
+      n0 += it.nb;
     }
   };
 
@@ -1154,19 +1151,17 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
   // The instruction is warpgroup-wide: all four warps of a warpgroup execute the same one, and the role
   // code sits inside the branch that issued it.
   if (!HAS_V) {
-    //   no V : 512 threads x 128 at launch; 384 x 152 + 128 x 56 = 65536; 3 x 152 + 56 = 512
+    //   no V : 640 threads x 96 at launch; 512 x 104 + 128 x 64 = 61440 = 640 x 96; 4 x 104 + 64 = 480
     if (warp < Cfg::kSoftmaxWarps) {
-      asm volatile("setmaxnreg.inc.sync.aligned.u32 152;\n");
+      asm volatile("setmaxnreg.inc.sync.aligned.u32 104;\n");
       if (POOL) pool_role(); else softmax_role();
     } else {
-      asm volatile("setmaxnreg.dec.sync.aligned.u32 56;\n");
+      asm volatile("setmaxnreg.dec.sync.aligned.u32 64;\n");
       if (warp == Cfg::kProducerWarp0) {
         if (lane == 0) producer_tma();
         __syncwarp();
       } else if (warp == kMmaWarp) {
-        mma_role(0);
-      } else if (Cfg::kIssuers == 2 && warp == kMmaWarp + 1) {
-        mma_role(1);
+        mma_role();
       }
     }
   } else if (warp < 8) {
