@@ -83,6 +83,14 @@ int kb200_topk_select(const float* scores, int64_t row_stride, int n_cols, const
                       const int32_t* k_row, int k_max, int32_t* out_idx, int64_t idx_stride,
                       int32_t* out_count, int64_t rows, void* stream);
 
+/* The same for the pooled scores of a decode step: row b * num_kv_heads + g has n = seq_lens[b] candidates, and its
+ * budget is the reference's (strategies/KascadeStrategy.py:127-129) with share = k / 100,
+ *   n <= 128 ? n : min(max(128, int(share * n)), n) - tile,
+ * capped at k_max. */
+int kb200_topk_select_decode(const float* scores, int64_t row_stride, int n_cols, const int32_t* seq_lens,
+                             int num_kv_heads, double share, int tile, int k_max, int32_t* out_idx,
+                             int64_t idx_stride, int32_t* out_count, int batch, void* stream);
+
 /* ---- paged decode (replaces kernels/flash_decoding/reuse_kascade_gqa_decode.py:50-134 and
  *      recompute_kascade_gqa_decode.py:49-315; the reference has no paged variant, README.md:135;
  *      the closest signature is reuse_kascade_gqa_decode_with_kvcache.py:160-171) --------------- */

@@ -22,7 +22,7 @@ DTYPES = {torch.float16: FP16, torch.bfloat16: BF16}
 FP8_TORCH = (torch.float8_e4m3fn, torch.uint8)   # an FP8 cache may be handed over as raw bytes
 
 EXPORTS = [
-    "kb200_init", "kb200_last_error", "kb200_abi_version", "kb200_topk_select",
+    "kb200_init", "kb200_last_error", "kb200_abi_version", "kb200_topk_select", "kb200_topk_select_decode",
     "kb200_decode_workspace_bytes", "kb200_decode_default_splits", "kb200_decode_sparse_paged",
     "kb200_decode_anchor_paged", "kb200_prefill_dense", "kb200_prefill_pool_scores",
     "kb200_prefill_sparse", "kb200_prefill_budgets", "kb200_selftest_umma", "kb200_read_status",
@@ -117,6 +117,7 @@ def load() -> C.CDLL:
         lib.kb200_init.argtypes = [C.c_int]
         vp, i64, i32, f32 = C.c_void_p, C.c_int64, C.c_int, C.c_float
         lib.kb200_topk_select.argtypes = [vp, i64, i32, vp, vp, i32, vp, i64, vp, i64, vp]
+        lib.kb200_topk_select_decode.argtypes = [vp, i64, i32, vp, i32, C.c_double, i32, i32, vp, i64, vp, i32, vp]
         lib.kb200_decode_sparse_paged.argtypes = [vp, i64, i64, C.POINTER(KvLayout), vp, i64, i64, vp,
                                                   i32, vp, f32, vp, vp, vp, C.c_size_t, i32, i32, i32,
                                                   i32, vp]
@@ -250,6 +251,23 @@ def topk_select(scores: torch.Tensor, n_valid: Optional[torch.Tensor], k_row: Op
                                  _ptr(n_valid), _ptr(k_row), k_max, _ptr(out_idx), out_idx.shape[-1],
                                  _ptr(out_count), rows, _stream()), "kb200_topk_select")
     _launched(1 if rows else 0)
+
+
+@_on_device_of(0)
+def topk_select_decode(scores: torch.Tensor, seq_lens: torch.Tensor, share: float, tile: int, k_max: int,
+                       out_idx: torch.Tensor, out_count: torch.Tensor, n_cols: int):
+    """topk_select over the pooled scores [B, G, row_stride] of a decode step; every row's number of candidates and
+    budget follow from seq_lens [B] int32 inside the kernel."""
+    lib = init(scores.device.index)
+    _want(scores, torch.float32, "scores")
+    _want(seq_lens, torch.int32, "seq_lens")
+    _want(out_idx, torch.int32, "out_idx")
+    B, G, stride = scores.shape
+    assert scores.is_contiguous() and out_idx.is_contiguous() and seq_lens.is_contiguous() and seq_lens.numel() == B
+    _check(lib.kb200_topk_select_decode(_ptr(scores), stride, n_cols, _ptr(seq_lens), G, share, tile, k_max,
+                                        _ptr(out_idx), out_idx.shape[-1], _ptr(out_count), B, _stream()),
+           "kb200_topk_select_decode")
+    _launched(1 if B else 0)
 
 
 @_on_device_of(0)

@@ -125,6 +125,20 @@ __device__ __forceinline__ uint32_t block_sum(TopkShared& sh, uint32_t v) {
   return t;
 }
 
+// Key budget of a decode step over a cache of n tokens (strategies/KascadeStrategy.py:127-129; up to 128 tokens
+// attend to everything), computed per row here: as tensors the budgets took a dozen element-wise launches per anchor
+// layer, more host time than the rest of the layer.
+struct DecodeBudget {
+  const int32_t* seq_lens;      // [rows / groups], or NULL: n_valid / k_row say how much to select
+  int groups;
+  double share;                 // k / 100
+  int tile;
+};
+__device__ __forceinline__ int decode_budget(const DecodeBudget& d, int n) {
+  if (n <= 128) return n;
+  return min(max(128, (int)(d.share * (double)n)), n) - d.tile;
+}
+
 #ifndef KB200_TOPK_MIN_CTAS
 #define KB200_TOPK_MIN_CTAS 2      // CTAs per SM the register allocation aims at (3, with a few spills, measured no faster)
 #endif
@@ -132,14 +146,20 @@ __global__ void __launch_bounds__(kTopkThreads, KB200_TOPK_MIN_CTAS)
 topk_select_kernel(const float* __restrict__ scores, int64_t row_stride, int n_cols,
                    const int32_t* __restrict__ n_valid, const int32_t* __restrict__ k_row, int k_max,
                    int32_t* __restrict__ out_idx, int64_t idx_stride, int32_t* __restrict__ out_count,
-                   int64_t rows) {
+                   int64_t rows, const DecodeBudget budget) {
   __shared__ TopkShared sh;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
   for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
-    int n = n_valid ? n_valid[row] : n_cols;
+    int n, k;
+    if (budget.seq_lens) {
+      n = budget.seq_lens[row / budget.groups];
+      k = min(decode_budget(budget, n), k_max);
+    } else {
+      n = n_valid ? n_valid[row] : n_cols;
+      k = k_row ? min(k_row[row], k_max) : k_max;
+    }
     n = max(0, min(n, n_cols));
-    int k = k_row ? min(k_row[row], k_max) : k_max;
     k = max(0, min(k, n));
     int32_t* out = out_idx + row * idx_stride;
     if (tid == 0 && out_count) out_count[row] = k;
@@ -570,11 +590,10 @@ extern "C" int kb200_prefill_budgets_ragged(int32_t* n_valid, int32_t* k_row, co
   return 0;
 }
 
-extern "C" int kb200_topk_select(const float* scores, int64_t row_stride, int n_cols,
-                                 const int32_t* n_valid, const int32_t* k_row, int k_max,
-                                 int32_t* out_idx, int64_t idx_stride, int32_t* out_count,
-                                 int64_t rows, void* stream) {
-  using namespace kb200;
+namespace kb200 {
+static int topk_launch(const float* scores, int64_t row_stride, int n_cols, const int32_t* n_valid,
+                       const int32_t* k_row, int k_max, int32_t* out_idx, int64_t idx_stride, int32_t* out_count,
+                       int64_t rows, const DecodeBudget& budget, void* stream) {
   KB_ENTRY(scores, "topk_select: scores");
   KB_REQUIRE(scores && out_idx, "topk_select: null pointer");
   KB_REQUIRE(rows >= 0 && n_cols >= 0 && k_max >= 0, "topk_select: negative size");
@@ -587,9 +606,29 @@ extern "C" int kb200_topk_select(const float* scores, int64_t row_stride, int n_
   if (rows == 0) return 0;
   int64_t grid = rows < (int64_t)sm_count() * 64 ? rows : (int64_t)sm_count() * 64;
   topk_select_kernel<<<(unsigned)grid, kTopkThreads, 0, (cudaStream_t)stream>>>(
-      scores, row_stride, n_cols, n_valid, k_row, k_max, out_idx, idx_stride, out_count, rows);
+      scores, row_stride, n_cols, n_valid, k_row, k_max, out_idx, idx_stride, out_count, rows, budget);
   KB_CHECK_LAUNCH("topk_select_kernel");
   return 0;
+}
+}  // namespace kb200
+
+extern "C" int kb200_topk_select(const float* scores, int64_t row_stride, int n_cols,
+                                 const int32_t* n_valid, const int32_t* k_row, int k_max,
+                                 int32_t* out_idx, int64_t idx_stride, int32_t* out_count,
+                                 int64_t rows, void* stream) {
+  return kb200::topk_launch(scores, row_stride, n_cols, n_valid, k_row, k_max, out_idx, idx_stride, out_count, rows,
+                            kb200::DecodeBudget{}, stream);
+}
+
+extern "C" int kb200_topk_select_decode(const float* scores, int64_t row_stride, int n_cols, const int32_t* seq_lens,
+                                        int num_kv_heads, double share, int tile, int k_max, int32_t* out_idx,
+                                        int64_t idx_stride, int32_t* out_count, int batch, void* stream) {
+  using namespace kb200;
+  KB_REQUIRE(seq_lens, "topk_select_decode: null pointer");
+  KB_REQUIRE(batch >= 0 && num_kv_heads > 0 && tile >= 0 && share >= 0.0 && share <= 1.0,
+             "topk_select_decode: batch %d, %d KV heads, tile %d, share %g", batch, num_kv_heads, tile, share);
+  return topk_launch(scores, row_stride, n_cols, nullptr, nullptr, k_max, out_idx, idx_stride, out_count,
+                     (int64_t)batch * num_kv_heads, DecodeBudget{seq_lens, num_kv_heads, share, tile}, stream);
 }
 
 extern "C" int kb200_prefill_budgets(int32_t* n_valid, int32_t* k_row, int batch, int num_kv_heads,

@@ -477,17 +477,10 @@ class EfficientKascadeStrategy(Strategy):
         return self._peer_fans[self._peer_copy]
 
     # -- decode ------------------------------------------------------------------------------------
-    def _decode_budgets(self, seq_lens: torch.Tensor, max_len: int):
-        """Per-sequence key budgets on the device (no sync): the reference formula for a cache of
-        seq_lens[b] keys; sequences of at most 128 keys attend to everything."""
-        lens = seq_lens.to(torch.float64)
-        kk = torch.clamp(torch.floor((self.k / 100) * lens), min=128.0)
-        kk = torch.minimum(kk, lens) - self.tile_size
-        kk = torch.where(lens <= 128, lens, kk).to(torch.int32)
-        # rows are as long as the largest per-sequence budget: the reference formula at max_len, and the
-        # "at most 128 keys: attend to everything" rule for the short sequences of a mixed batch
-        kmax = max_len if max_len <= 128 else max(topk_budget(self.k, max_len, self.tile_size), 128)
-        return kk, max(kmax, 1)
+    def _decode_row_length(self, max_len: int) -> int:
+        """Length of a decode step's index rows: the largest budget of any sequence, i.e. the reference formula at max_len
+        and the "at most 128 keys: attend to everything" rule for the short sequences of a mixed batch."""
+        return max(max_len if max_len <= 128 else max(topk_budget(self.k, max_len, self.tile_size), 128), 1)
 
     @staticmethod
     def _splits(B: int, G: int, keys_max: int, raggedness: float, dev) -> int:
@@ -522,13 +515,11 @@ class EfficientKascadeStrategy(Strategy):
                                     lse2, ws, splits_a)
             if dense_only:
                 return out
-            k_row, kmax = self._decode_budgets(seq_lens, max_len)
-            self._dec_kmax = kmax
+            self._dec_kmax = kmax = self._decode_row_length(max_len)
             self._dec_idx = self._scratch("dec_idx", (B, G, kmax), torch.int32, dev)
             self._dec_count = self._scratch("dec_count", (B, G), torch.int32, dev)
-            n_valid = seq_lens.view(B, 1).expand(B, G).contiguous()
-            k_rows = k_row.view(B, 1).expand(B, G).contiguous()
-            nat.topk_select(pooled, n_valid, k_rows, kmax, self._dec_idx, self._dec_count, n_cols=max_len)
+            nat.topk_select_decode(pooled, seq_lens, self.k / 100, self.tile_size, kmax, self._dec_idx, self._dec_count,
+                                   n_cols=max_len)
             if layer == 0:
                 return out
             head_map = None

@@ -133,3 +133,39 @@ def test_rejects_bad_arguments():
     out = torch.zeros(2, 4, dtype=torch.int32, device=dev)
     with pytest.raises(nat.KascadeNativeError):
         nat.topk_select(s, None, None, 4, out, None)
+
+
+@pytest.mark.parametrize("share", [0.0, 0.05, 0.1, 0.2, 1.0])
+def test_decode_budgets_inside_the_kernel_select_what_the_tensors_did(share):
+    """topk_select_decode derives a row's candidates and budget from seq_lens; the general entry given them as tensors
+    (computed here in 64 bits) selects the same positions.  Lengths: empty, the edges of the 128-key rule, a length whose
+    share falls below the tile, one whose product with the share is a whole number, one beyond n_cols, the largest."""
+    from kascade_b200 import _native as nat
+    dev = torch.device("cuda")
+    lens = torch.tensor([0, 1, 127, 128, 129, 161, 1279, 1280, 4097, 5000, 9000, 70001], dtype=torch.int32)
+    B, G, n_cols, tile = len(lens), 3, 70000, 32
+    scores = torch.rand(B, G, n_cols, generator=torch.Generator().manual_seed(3)).to(dev)
+    n = lens.double()
+    k = torch.minimum(torch.clamp(torch.floor(share * n), min=128.0), n) - tile
+    k = torch.where(n <= 128, n, k).to(torch.int32)
+    k_max = 7000
+    out = [torch.full((B, G, k_max), -7, dtype=torch.int32, device=dev) for _ in range(2)]
+    cnt = [torch.full((B, G), -1, dtype=torch.int32, device=dev) for _ in range(2)]
+    nat.topk_select(scores, lens.to(dev).view(B, 1).expand(B, G).contiguous(), k.to(dev).view(B, 1).expand(B, G).contiguous(),
+                    k_max, out[0], cnt[0], n_cols=n_cols)
+    nat.topk_select_decode(scores, lens.to(dev), share, tile, k_max, out[1], cnt[1], n_cols=n_cols)
+    assert torch.equal(cnt[0], cnt[1]) and torch.equal(out[0], out[1])
+    assert cnt[1][:, 0].tolist() == [min(int(a), int(b), n_cols, k_max) for a, b in zip(k, lens)]
+
+
+def test_decode_selection_rejects_bad_arguments():
+    from kascade_b200 import _native as nat
+    dev = torch.device("cuda")
+    scores = torch.zeros(2, 2, 64, device=dev)
+    out = torch.zeros(2, 2, 64, dtype=torch.int32, device=dev)
+    cnt = torch.zeros(2, 2, dtype=torch.int32, device=dev)
+    lens = torch.full((2,), 64, dtype=torch.int32, device=dev)
+    with pytest.raises(nat.KascadeNativeError, match="share"):
+        nat.topk_select_decode(scores, lens, 1.5, 32, 64, out, cnt, n_cols=64)
+    with pytest.raises(nat.KascadeNativeError, match="seq_lens"):
+        nat.topk_select_decode(scores, lens.long(), 0.1, 32, 64, out, cnt, n_cols=64)
