@@ -59,6 +59,7 @@ int sm_count();
 // per-module init hooks (raise dynamic shared memory limits); defined in the kernel files
 int init_decode();
 int init_prefill();
+int init_topk();
 int init_selftest();
 
 }  // namespace kb200

@@ -20,6 +20,13 @@
 //   4. The last pass writes the selected positions of every warp's piece in index order, with warp-local prefix
 //      sums only, taking ties at the threshold from the lowest index upwards.
 // The row is read from HBM once; the later passes find it in L1 / L2.
+//
+// A few long rows (the anchor layers of a decode step with a handful of sequences) would leave most SMs idle: a
+// cluster of 2, 4 or 8 CTAs then takes a row together.  Each takes the whole sample and comes to the same bracket,
+// streams its own piece of the row, and the lists of all of them (a few thousand keys) are gathered over distributed
+// shared memory, so that the radix select needs no exchange either.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace kb200 {
@@ -31,6 +38,7 @@ constexpr int kTopkBins = 1 << kDigit;                            // 9-bit digit
 constexpr int kCandCap = 8192;                            // keys the candidate lists hold, one list per warp
 constexpr int kWarpList = kCandCap / kTopkWarps;          // 512
 constexpr int kListRow = 4096;                            // rows up to this length are selected from directly
+constexpr int kTopkMergedBytes = kCandCap * 4;            // dynamic shared memory of a cluster's CTA
 constexpr int kTopkUnroll = 4;                            // 16-byte loads a lane keeps in flight in the streaming passes
 
 // order-preserving map float -> uint32 (larger float <=> larger key)
@@ -56,6 +64,9 @@ struct TopkShared {
   uint32_t red[kTopkWarps], red2[kTopkWarps];
   uint32_t warp_gt[kTopkWarps], warp_eq[kTopkWarps], list_len[kTopkWarps];
   uint32_t digit, remaining;
+  uint32_t cta_gt, cta_cand, cta_max_list;               // clusters: scores above hi_key, list entries, longest list
+  uint32_t cta_above, cta_equal;                         // clusters: scores above / at the threshold in this CTA's piece
+  uint32_t list_at[8 * kTopkWarps];                      // clusters: where each list starts in the gathered one
 };
 
 // Bin d of sh.hist with  count(bins > d) < r <= count(bins >= d)  (1 <= r <= total); every thread gets d and
@@ -142,15 +153,19 @@ __device__ __forceinline__ int decode_budget(const DecodeBudget& d, int n) {
 #ifndef KB200_TOPK_MIN_CTAS
 #define KB200_TOPK_MIN_CTAS 2      // CTAs per SM the register allocation aims at (3, with a few spills, measured no faster)
 #endif
+template <int C>                       // CTAs that share a row (a cluster of C)
 __global__ void __launch_bounds__(kTopkThreads, KB200_TOPK_MIN_CTAS)
 topk_select_kernel(const float* __restrict__ scores, int64_t row_stride, int n_cols,
                    const int32_t* __restrict__ n_valid, const int32_t* __restrict__ k_row, int k_max,
                    int32_t* __restrict__ out_idx, int64_t idx_stride, int32_t* __restrict__ out_count,
                    int64_t rows, const DecodeBudget budget) {
+  namespace cg = cooperative_groups;
   __shared__ TopkShared sh;
+  extern __shared__ uint32_t merged[];                    // C > 1: the lists of all CTAs of the cluster
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rank = C > 1 ? (int)cg::this_cluster().block_rank() : 0;
 
-  for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
+  for (int64_t row = blockIdx.x / C; row < rows; row += gridDim.x / C) {
     int n, k;
     if (budget.seq_lens) {
       n = budget.seq_lens[row / budget.groups];
@@ -162,17 +177,17 @@ topk_select_kernel(const float* __restrict__ scores, int64_t row_stride, int n_c
     n = max(0, min(n, n_cols));
     k = max(0, min(k, n));
     int32_t* out = out_idx + row * idx_stride;
-    if (tid == 0 && out_count) out_count[row] = k;
+    if (tid == 0 && rank == 0 && out_count) out_count[row] = k;
     if (k == 0) continue;
     if (k == n) {  // every candidate is selected
-      for (int i = tid; i < n; i += kTopkThreads) out[i] = i;
+      for (int i = rank * kTopkThreads + tid; i < n; i += C * kTopkThreads) out[i] = i;
       continue;
     }
     const float4* row4 = reinterpret_cast<const float4*>(scores + row * row_stride);
     const int n4 = (n + 3) >> 2;
-    // warp w owns the 16-byte pieces [w_begin, w_end) of the row
-    const int seg4 = (n4 + kTopkWarps - 1) / kTopkWarps;
-    const int w_begin = min(warp * seg4, n4), w_end = min(w_begin + seg4, n4);
+    // every warp (of the cluster) owns the 16-byte pieces [w_begin, w_end) of the row
+    const int seg4 = (n4 + C * kTopkWarps - 1) / (C * kTopkWarps);
+    const int w_begin = min((rank * kTopkWarps + warp) * seg4, n4), w_end = min(w_begin + seg4, n4);
     const int w_iters = (w_end - w_begin + 31) >> 5;
 
     // ---- 1. bracket [lo_key, hi_key] of the k-th largest key from a sample ----------------------------
@@ -333,15 +348,61 @@ topk_select_kernel(const float* __restrict__ scores, int64_t row_stride, int n_c
     const uint32_t my_gt_hi = cnt_gt;                     // scores of this warp's piece above hi_key
     if (lane != 0) cnt_gt = 0;
     if (lane == 0) sh.list_len[warp] = my_cand;
-    const uint32_t n_gt = block_sum(sh, cnt_gt);          // (its barriers also publish the lists and their lengths)
-    const uint32_t n_cand = warps_sum(sh.list_len);
-    const bool fits = warps_max(sh.list_len) <= (uint32_t)kWarpList;
+    uint32_t n_gt = block_sum(sh, cnt_gt);                // (its barriers also publish the lists and their lengths)
+    uint32_t n_cand = warps_sum(sh.list_len);
+    bool fits = warps_max(sh.list_len) <= (uint32_t)kWarpList;
+    if constexpr (C > 1) {
+      cg::cluster_group cluster = cg::this_cluster();
+      const uint32_t longest = warps_max(sh.list_len);
+      if (tid == 0) { sh.cta_gt = n_gt; sh.cta_cand = n_cand; sh.cta_max_list = longest; }
+      cluster.sync();
+      n_gt = n_cand = 0;
+#pragma unroll
+      for (int r = 0; r < C; ++r) {
+        const TopkShared* peer = cluster.map_shared_rank(&sh, r);
+        n_gt += peer->cta_gt;
+        n_cand += peer->cta_cand;
+        fits = fits && peer->cta_max_list <= (uint32_t)kWarpList;
+      }
+      fits = fits && n_cand <= (uint32_t)kCandCap;
+      if (fits) {                                         // (the same for the whole cluster)
+        if (warp == 0) {                                  // C / 2 lists per lane
+          constexpr int kPer = C * kTopkWarps / 32;
+          uint32_t len[kPer], sum = 0;
+#pragma unroll
+          for (int i = 0; i < kPer; ++i) {
+            const int l = lane * kPer + i;
+            len[i] = cluster.map_shared_rank(&sh, l / kTopkWarps)->list_len[l % kTopkWarps];
+            sum += len[i];
+          }
+          uint32_t incl = sum;
+#pragma unroll
+          for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, off);
+            if (lane >= off) incl += v;
+          }
+          uint32_t at = incl - sum;
+#pragma unroll
+          for (int i = 0; i < kPer; ++i) { sh.list_at[lane * kPer + i] = at; at += len[i]; }
+        }
+        __syncthreads();
+        for (int l = warp; l < C * kTopkWarps; l += kTopkWarps) {
+          const uint32_t begin = sh.list_at[l], end = l + 1 < C * kTopkWarps ? sh.list_at[l + 1] : n_cand;
+          const uint32_t* src = cluster.map_shared_rank(&sh, l / kTopkWarps)->cand + (l % kTopkWarps) * kWarpList;
+          for (uint32_t i = lane; i < end - begin; i += 32) merged[begin + i] = src[i];
+        }
+        __syncthreads();
+      }
+    }
+    // the candidates: every warp walks its own list, or the CTA the gathered one
+    const uint32_t* const cand_list = C > 1 ? merged : my_list;
+    const uint32_t cand_n = C > 1 ? n_cand : my_cand, cand_first = C > 1 ? tid : lane, cand_step = C > 1 ? kTopkThreads : 32;
 
     if (!sampled) {
       // the whole row is the list: its own key range instead of all 32 bits, so that the first digit spreads
       uint32_t cmin = 0xFFFFFFFFu, cmax = 0u;
       if (fits)
-        for (uint32_t i = lane; i < my_cand; i += 32) { cmin = min(cmin, my_list[i]); cmax = max(cmax, my_list[i]); }
+        for (uint32_t i = cand_first; i < cand_n; i += cand_step) { cmin = min(cmin, cand_list[i]); cmax = max(cmax, cand_list[i]); }
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) {
         cmin = min(cmin, __shfl_xor_sync(0xFFFFFFFFu, cmin, off));
@@ -367,8 +428,8 @@ topk_select_kernel(const float* __restrict__ scores, int64_t row_stride, int n_c
         const uint32_t dmask = (1u << (hb - shift)) - 1u;
         for (int i = tid; i < kTopkBins; i += kTopkThreads) sh.hist[i] = 0;
         __syncthreads();
-        for (uint32_t i = lane; i < my_cand; i += 32) {    // every warp bins its own list
-          const uint32_t v = my_list[i] - lo_key;
+        for (uint32_t i = cand_first; i < cand_n; i += cand_step) {
+          const uint32_t v = cand_list[i] - lo_key;
           if ((v & mask) == prefix) atomicAdd(&sh.hist[(v >> shift) & dmask], 1u);
         }
         __syncthreads();
@@ -470,6 +531,17 @@ topk_select_kernel(const float* __restrict__ scores, int64_t row_stride, int n_c
       gt_before = g;
       eq_before = q;
     }
+    if constexpr (C > 1) {                                // ... and in the pieces of the CTAs before this one
+      cg::cluster_group cluster = cg::this_cluster();
+      const uint32_t above = warps_sum(sh.warp_gt), equal = warps_sum(sh.warp_eq);
+      if (tid == 0) { sh.cta_above = above; sh.cta_equal = equal; }
+      cluster.sync();
+      for (int r = 0; r < rank; ++r) {
+        const TopkShared* peer = cluster.map_shared_rank(&sh, r);
+        gt_before += peer->cta_above;
+        eq_before += peer->cta_equal;
+      }
+    }
     // ---- 4. write the selected positions of this warp's piece, in index order -----------------------------
     for (int it0 = 0; it0 < w_iters; it0 += kTopkUnroll) {
       float4 xs[kTopkUnroll];
@@ -534,7 +606,8 @@ topk_select_kernel(const float* __restrict__ scores, int64_t row_stride, int n_c
         }
       }
     }
-    __syncthreads();                                      // the shared arrays are reused by the next row
+    if constexpr (C > 1) cg::this_cluster().sync();       // ... and read by the other CTAs until here
+    else __syncthreads();                                 // the shared arrays are reused by the next row
   }
 }
 
@@ -591,6 +664,44 @@ extern "C" int kb200_prefill_budgets_ragged(int32_t* n_valid, int32_t* k_row, co
 }
 
 namespace kb200 {
+template <int C>
+static cudaError_t topk_launch_cluster(const float* scores, int64_t row_stride, int n_cols, const int32_t* n_valid,
+                                       const int32_t* k_row, int k_max, int32_t* out_idx, int64_t idx_stride,
+                                       int32_t* out_count, int64_t rows, const DecodeBudget& budget, cudaStream_t st) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(rows * C));
+  cfg.blockDim = dim3(kTopkThreads);
+  cfg.dynamicSmemBytes = kTopkMergedBytes;
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = C;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, topk_select_kernel<C>, scores, row_stride, n_cols, n_valid, k_row, k_max, out_idx,
+                            idx_stride, out_count, rows, budget);
+}
+
+// CTAs per row: doubled while all rows together leave an SM for each CTA and a CTA keeps at least 4096 scores; below
+// that, and for rows under 16384, its fixed phases (the sample, the lists) cost more than a shorter piece saves.
+// Measured, us with one CTA / a cluster: 8 rows of 16384 / 32768 / 131072 scores 17.2 / 25.4 / 69.9 -> 15.2 / 18.5 / 27.1,
+// 32 x 65536 41.4 -> 23.7 (29.2 with two CTAs on an SM), 64 x 32768 25.7 -> 21.1; 128 x 16384 17.8 -> 20.3 with two, 8 x 8192
+// 13.3 -> 13.7: not taken.
+static int topk_cluster(int64_t rows, int n_cols) {
+  int c = 1;
+  if (n_cols < 16384) return c;
+  while (c < 8 && rows * (2 * c) <= sm_count() && n_cols / (2 * c) >= 4096) c *= 2;
+  return c;
+}
+
+int init_topk() {
+  KB_CUDA(cudaFuncSetAttribute(topk_select_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTopkMergedBytes));
+  KB_CUDA(cudaFuncSetAttribute(topk_select_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTopkMergedBytes));
+  KB_CUDA(cudaFuncSetAttribute(topk_select_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTopkMergedBytes));
+  return 0;
+}
+
 static int topk_launch(const float* scores, int64_t row_stride, int n_cols, const int32_t* n_valid,
                        const int32_t* k_row, int k_max, int32_t* out_idx, int64_t idx_stride, int32_t* out_count,
                        int64_t rows, const DecodeBudget& budget, void* stream) {
@@ -604,10 +715,24 @@ static int topk_launch(const float* scores, int64_t row_stride, int n_cols, cons
   KB_REQUIRE(idx_stride >= (int64_t)k_max, "topk_select: idx_stride (%lld) smaller than k_max (%d)",
              (long long)idx_stride, k_max);
   if (rows == 0) return 0;
-  int64_t grid = rows < (int64_t)sm_count() * 64 ? rows : (int64_t)sm_count() * 64;
-  topk_select_kernel<<<(unsigned)grid, kTopkThreads, 0, (cudaStream_t)stream>>>(
-      scores, row_stride, n_cols, n_valid, k_row, k_max, out_idx, idx_stride, out_count, rows, budget);
-  KB_CHECK_LAUNCH("topk_select_kernel");
+  cudaStream_t st = (cudaStream_t)stream;
+  switch (topk_cluster(rows, n_cols)) {
+    case 8:
+      KB_CUDA(topk_launch_cluster<8>(scores, row_stride, n_cols, n_valid, k_row, k_max, out_idx, idx_stride, out_count, rows, budget, st));
+      break;
+    case 4:
+      KB_CUDA(topk_launch_cluster<4>(scores, row_stride, n_cols, n_valid, k_row, k_max, out_idx, idx_stride, out_count, rows, budget, st));
+      break;
+    case 2:
+      KB_CUDA(topk_launch_cluster<2>(scores, row_stride, n_cols, n_valid, k_row, k_max, out_idx, idx_stride, out_count, rows, budget, st));
+      break;
+    default: {
+      const int64_t grid = rows < (int64_t)sm_count() * 64 ? rows : (int64_t)sm_count() * 64;
+      topk_select_kernel<1><<<(unsigned)grid, kTopkThreads, 0, st>>>(scores, row_stride, n_cols, n_valid, k_row, k_max, out_idx,
+                                                                     idx_stride, out_count, rows, budget);
+      KB_CHECK_LAUNCH("topk_select_kernel");
+    }
+  }
   return 0;
 }
 }  // namespace kb200

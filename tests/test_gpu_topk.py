@@ -169,3 +169,41 @@ def test_decode_selection_rejects_bad_arguments():
         nat.topk_select_decode(scores, lens, 1.5, 32, 64, out, cnt, n_cols=64)
     with pytest.raises(nat.KascadeNativeError, match="seq_lens"):
         nat.topk_select_decode(scores, lens.long(), 0.1, 32, 64, out, cnt, n_cols=64)
+
+
+@pytest.mark.parametrize("rows,n", [(1, 8191), (1, 8192), (1, 16384), (3, 32768), (8, 131071), (37, 33000), (38, 33000), (74, 16400),
+                                    (75, 16400), (148, 9000), (149, 9000)])
+@pytest.mark.parametrize("kind", ["smooth", "ties", "steps"])
+def test_rows_shared_by_a_cluster(rows, n, kind):
+    """Few long rows are split over the CTAs of a cluster (2, 4 or 8, by rows and columns).  The selection is exact, so it
+    equals a stable sort's, ties from the lowest index, whatever the number of CTAs: also where the sample's bracket
+    fails (`ties`: half of the row has one value; `steps`: four values) and where single rows are short, empty or
+    selected as a whole."""
+    from kascade_b200 import _native as nat
+    dev = torch.device("cuda")
+    g = torch.Generator().manual_seed(rows * 7 + n)
+    s = torch.rand(rows, n, generator=g) ** 6
+    if kind == "ties":
+        s[torch.rand(rows, n, generator=g) < 0.5] = 0.125
+    elif kind == "steps":
+        s = torch.floor(s * 4) / 4
+    stride = (n + 3) // 4 * 4
+    scores = torch.nn.functional.pad(s, (0, stride - n), value=9.0).to(dev)
+    n_valid = torch.full((rows,), n, dtype=torch.int32)
+    k_row = torch.full((rows,), max(128, n // 10), dtype=torch.int32)
+    if rows > 2:                                          # a short row, an empty one, one that is selected as a whole
+        n_valid[0], n_valid[1], k_row[2] = 700, 0, n
+    out = torch.full((rows, n), -7, dtype=torch.int32, device=dev)
+    cnt = torch.full((rows,), -1, dtype=torch.int32, device=dev)
+    nat.topk_select(scores, n_valid.to(dev), k_row.to(dev), n, out, cnt, n_cols=n)
+    order = torch.sort(scores[:, :n], dim=-1, descending=True, stable=True).indices
+    for r in range(rows):
+        k = min(int(k_row[r]), int(n_valid[r]))
+        assert int(cnt[r]) == k
+        if int(n_valid[r]) == n:
+            want = order[r, :k].sort().values
+        else:
+            m = int(n_valid[r])
+            want = torch.sort(scores[r, :m], descending=True, stable=True).indices[:k].sort().values
+        assert torch.equal(out[r, :k].long(), want), f"row {r}"
+        assert (out[r, k:] == -7).all()
