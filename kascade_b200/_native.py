@@ -6,6 +6,7 @@ missing or a call is rejected, a ``KascadeNativeError`` is raised.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import os
 from typing import Optional
 
@@ -161,6 +162,8 @@ def _check(rc: int, what: str):
 
 
 def init(device: Optional[int] = None) -> C.CDLL:
+    if device in _inited and _lib is not None:      # every call of a step comes through here: nothing but the look-up
+        return _lib
     lib = load()
     if not torch.cuda.is_available():
         raise KascadeNativeError("kascade_b200 needs a CUDA device (sm_100a); none is visible")
@@ -197,14 +200,12 @@ def _on_device_of(arg_index: int):
     state (kernel attributes, the built-in decode scratch) by it; without this a caller whose current device
     differs from the tensors' would launch on the wrong GPU."""
     def deco(fn):
-        import functools
-
         @functools.wraps(fn)
         def wrapped(*args, **kwargs):
             t = args[arg_index]
             if not t.is_cuda:
                 raise KascadeNativeError(f"{fn.__name__}: expected CUDA tensors, got one on {t.device}")
-            if t.device.index == torch.cuda.current_device():
+            if t.get_device() == torch._C._cuda_getDevice():     # (a CUDA tensor exists: the runtime is up)
                 return fn(*args, **kwargs)
             with torch.cuda.device(t.device):
                 return fn(*args, **kwargs)
@@ -212,12 +213,13 @@ def _on_device_of(arg_index: int):
     return deco
 
 
-def _stream() -> C.c_void_p:
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+def _stream() -> int:
+    """cudaStream_t of the current device's current stream (read as a handle, without building a torch.cuda.Stream)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
-def _ptr(t: Optional[torch.Tensor]) -> C.c_void_p:
-    return C.c_void_p(0 if t is None else t.data_ptr())
+def _ptr(t: Optional[torch.Tensor]) -> int:
+    return 0 if t is None else t.data_ptr()
 
 
 def _want_opt(t: Optional[torch.Tensor], dtype, name: str):
@@ -242,7 +244,7 @@ def _half_code(t: torch.Tensor, name: str) -> int:
 def topk_select(scores: torch.Tensor, n_valid: Optional[torch.Tensor], k_row: Optional[torch.Tensor],
                 k_max: int, out_idx: torch.Tensor, out_count: Optional[torch.Tensor], n_cols: Optional[int] = None):
     """scores [..., row_stride] fp32 (last dim contiguous, rows equally spaced), out_idx [..., idx_stride]."""
-    lib = init(scores.device.index)
+    lib = init(scores.get_device())
     _want(scores, torch.float32, "scores")
     _want(out_idx, torch.int32, "out_idx")
     rows = scores.numel() // scores.shape[-1]
@@ -258,7 +260,7 @@ def topk_select_decode(scores: torch.Tensor, seq_lens: torch.Tensor, share: floa
                        out_idx: torch.Tensor, out_count: torch.Tensor, n_cols: int):
     """topk_select over the pooled scores [B, G, row_stride] of a decode step; every row's number of candidates and
     budget follow from seq_lens [B] int32 inside the kernel."""
-    lib = init(scores.device.index)
+    lib = init(scores.get_device())
     _want(scores, torch.float32, "scores")
     _want(seq_lens, torch.int32, "seq_lens")
     _want(out_idx, torch.int32, "out_idx")
@@ -272,7 +274,7 @@ def topk_select_decode(scores: torch.Tensor, seq_lens: torch.Tensor, share: floa
 
 @_on_device_of(0)
 def prefill_budgets(n_valid, k_row, batch, groups, tiles, k_max, pct, rolling):
-    lib = init(n_valid.device.index)
+    lib = init(n_valid.get_device())
     _check(lib.kb200_prefill_budgets(_ptr(n_valid), _ptr(k_row), batch, groups, tiles, k_max, float(pct),
                                      int(bool(rolling)), _stream()), "kb200_prefill_budgets")
     _launched(1)
@@ -280,7 +282,7 @@ def prefill_budgets(n_valid, k_row, batch, groups, tiles, k_max, pct, rolling):
 
 @_on_device_of(0)
 def prefill_budgets_ragged(n_valid, k_row, seq_len, batch, groups, tiles, k_cap, pct, rolling):
-    lib = init(n_valid.device.index)
+    lib = init(n_valid.get_device())
     _want(seq_len, torch.int32, "seq_len")
     _check(lib.kb200_prefill_budgets_ragged(_ptr(n_valid), _ptr(k_row), _ptr(seq_len), batch, groups, tiles, k_cap,
                                             float(pct), int(bool(rolling)), _stream()), "kb200_prefill_budgets_ragged")
@@ -319,13 +321,14 @@ def kv_layout_paged(k_cache: torch.Tensor, v_cache: Optional[torch.Tensor], bloc
                                  0 if v_scale is None else v_scale.data_ptr(), 0, k_scale.stride(0), k_scale.stride(1)),
                         k_cache, v_cache, block_table, k_scale, v_scale)
     code = _half_code(k_cache, "k_cache")
-    assert k_cache.dim() == 4 and k_cache.stride(3) == 1
+    st = k_cache.stride()
+    assert len(st) == 4 and st[3] == 1
     assert block_table.dtype == torch.int32 and block_table.stride(1) == 1
     if v_cache is not None:
-        assert v_cache.shape == k_cache.shape and v_cache.stride() == k_cache.stride() and v_cache.dtype == k_cache.dtype
-    return _holding(KvLayout(k_cache.data_ptr(), 0 if v_cache is None else v_cache.data_ptr(), 0, k_cache.stride(0),
-                             k_cache.stride(1), k_cache.stride(2), block_table.data_ptr(), block_table.stride(0),
-                             k_cache.shape[1], code), k_cache, v_cache, block_table)
+        assert v_cache.shape == k_cache.shape and v_cache.stride() == st and v_cache.dtype == k_cache.dtype
+    return _holding(KvLayout(k_cache.data_ptr(), 0 if v_cache is None else v_cache.data_ptr(), 0, st[0], st[1], st[2],
+                             block_table.data_ptr(), block_table.stride(0), k_cache.shape[1], code),
+                    k_cache, v_cache, block_table)
 
 
 def kv_layout_contiguous(k: torch.Tensor, v: Optional[torch.Tensor], page_size: int = 16,
@@ -343,11 +346,12 @@ def kv_layout_contiguous(k: torch.Tensor, v: Optional[torch.Tensor], page_size: 
                                  0 if v_scale is None else v_scale.data_ptr(), k_scale.stride(0), k_scale.stride(2),
                                  k_scale.stride(1)), k, v, k_scale, v_scale)
     code = _half_code(k, "k")
-    assert k.dim() == 4 and k.stride(3) == 1
+    st = k.stride()
+    assert len(st) == 4 and st[3] == 1
     if v is not None:
-        assert v.shape == k.shape and v.stride() == k.stride() and v.dtype == k.dtype
-    return _holding(KvLayout(k.data_ptr(), 0 if v is None else v.data_ptr(), k.stride(0), k.stride(2) * page_size,
-                             k.stride(2), k.stride(1), 0, 0, page_size, code), k, v)
+        assert v.shape == k.shape and v.stride() == st and v.dtype == k.dtype
+    return _holding(KvLayout(k.data_ptr(), 0 if v is None else v.data_ptr(), st[0], st[2] * page_size, st[2], st[1], 0, 0,
+                             page_size, code), k, v)
 
 
 def kv_layout_rows(k: torch.Tensor, v: Optional[torch.Tensor], row_table: torch.Tensor) -> KvLayout:
@@ -368,16 +372,20 @@ def decode_workspace(batch: int, heads: int, splits: int, device) -> torch.Tenso
     return torch.empty(max(n, 16), dtype=torch.uint8, device=device)
 
 
-def decode_default_splits(batch: int, groups: int, max_keys: int) -> int:
-    init()
-    return load().kb200_decode_default_splits(batch, groups, max_keys)
+def decode_default_splits(batch: int, groups: int, max_keys: int, device: Optional[int] = None) -> int:
+    return init(device).kb200_decode_default_splits(batch, groups, max_keys)
+
+
+@functools.lru_cache(maxsize=None)
+def sm_count(device: int) -> int:
+    return torch.cuda.get_device_properties(device).multi_processor_count
 
 
 @_on_device_of(0)
 def decode_sparse_paged(q, kv: KvLayout, topk_idx, topk_count, k_max, head_map, scale, out, lse2=None,
                         workspace=None, num_splits=0):
     """q [B,H,D] fp16; topk_idx [B,G,kstride] int32; out [B,H,D] fp16 contiguous."""
-    lib = init(q.device.index)
+    lib = init(q.get_device())
     if _half_code(q, "q") != (FP16 if kv.dtype == FP8_E4M3 else kv.dtype):
         raise KascadeNativeError(f"q is {q.dtype} but the KV cache has dtype code {kv.dtype} (an FP8 cache takes fp16 q)")
     _want(out, q.dtype, "out")
@@ -405,7 +413,7 @@ def decode_sparse_paged_noalloc(q, kv: KvLayout, topk_idx, topk_count, k_max, he
     """Same result as decode_sparse_paged, for callers that cannot allocate or pass a workspace: the split
     partials live in a fixed array inside the library (batch * heads * splits <= NOALLOC_MAX_SLOTS).
     Calls that overlap on the GPU race on that array; the first call on a device belongs in set-up."""
-    lib = init(q.device.index)
+    lib = init(q.get_device())
     if _half_code(q, "q") != (FP16 if kv.dtype == FP8_E4M3 else kv.dtype):
         raise KascadeNativeError(f"q is {q.dtype} but the KV cache has dtype code {kv.dtype} (an FP8 cache takes fp16 q)")
     _want(out, q.dtype, "out")
@@ -426,7 +434,7 @@ def decode_sparse_paged_noalloc(q, kv: KvLayout, topk_idx, topk_count, k_max, he
 def decode_anchor_paged(q, kv: KvLayout, seq_lens, max_seq_len, scale, logits, pooled, out, lse2,
                         workspace=None, num_splits=0):
     """q [B,H,D]; logits [B,H,stride] fp32; pooled [B,G,stride] fp32; out [B,H,D] fp16 or None."""
-    lib = init(q.device.index)
+    lib = init(q.get_device())
     if _half_code(q, "q") != (FP16 if kv.dtype == FP8_E4M3 else kv.dtype):
         raise KascadeNativeError(f"q is {q.dtype} but the KV cache has dtype code {kv.dtype} (an FP8 cache takes fp16 q)")
     _want_opt(out, q.dtype, "out")
@@ -447,8 +455,9 @@ def decode_anchor_paged(q, kv: KvLayout, seq_lens, max_seq_len, scale, logits, p
 def act_layout(x: torch.Tensor) -> ActLayout:
     """x indexed [B, L, heads, D] (any strides, D contiguous)."""
     code = _half_code(x, "activation")
-    assert x.dim() == 4 and x.stride(3) == 1 and x.shape[3] == HEAD_DIM
-    return ActLayout(x.data_ptr(), x.stride(0), x.stride(1), x.stride(2), code)
+    st = x.stride()
+    assert len(st) == 4 and st[3] == 1 and x.shape[3] == HEAD_DIM
+    return ActLayout(x.data_ptr(), st[0], st[1], st[2], code)
 
 
 @_on_device_of(0)
@@ -456,7 +465,7 @@ def prefill_dense(q, k, v, scale, out, lse2, fanout: Optional[OutFanout] = None,
     """q [B,L,H,D], k/v [B,L,G,D] (views allowed); out [B,L,H,D] fp16 contiguous or None; lse2 [B,L,H] fp32 or None.
     With `fanout` (see out_fanout) the rows go into several [B,L,total_heads,D] buffers instead of `out`; with
     `ragged` (see ragged()) every sequence has its own first row and length inside its slot of L rows."""
-    lib = init(q.device.index)
+    lib = init(q.get_device())
     B, L, H, _ = q.shape
     G = k.shape[2]
     ql, kl = act_layout(q), act_layout(k)
@@ -485,7 +494,7 @@ def prefill_dense(q, k, v, scale, out, lse2, fanout: Optional[OutFanout] = None,
 @_on_device_of(0)
 def prefill_pool_scores(q, k, lse2, scale, pooled, ragged: Optional[Ragged] = None):
     """pooled [B,G,T,row_stride] fp32 contiguous."""
-    lib = init(q.device.index)
+    lib = init(q.get_device())
     B, L, H, _ = q.shape
     G = k.shape[2]
     ql, kl = act_layout(q), act_layout(k)
@@ -508,7 +517,7 @@ def prefill_sparse(q, k, v, tile_idx, tile_count, head_map, scale, out, lse2=Non
                    ragged: Optional[Ragged] = None):
     """tile_idx [B,G,T,kstride] int32, tile_count [B,G,T] int32, out [B,L,H,D] fp16 contiguous.
     With `fanout` (see out_fanout) the rows go into several [B,L,total_heads,D] buffers instead of `out`."""
-    lib = init(q.device.index)
+    lib = init(q.get_device())
     B, L, H, _ = q.shape
     G = k.shape[2]
     ql, kl, vl = act_layout(q), act_layout(k), act_layout(v)
@@ -544,7 +553,7 @@ def kv_write(q_in, q_out, k_new, v_new, start_pos, n_new, kv: KvLayout, q_gain=N
     """q_in [B,T,H,D] (or None), k_new / v_new [B,T,G,D] views, all fp16 or all bf16 like the cache and the gains;
     start_pos [B] int32; n_new [B] int32 or None; kv: the cache to append to (kv_layout_paged /
     kv_layout_contiguous); inv_freq [D/2] fp32 or None."""
-    lib = init(k_new.device.index)
+    lib = init(k_new.get_device())
     B, T, G, _ = k_new.shape
     kl, vl = act_layout(k_new), act_layout(v_new)
     ql = act_layout(q_in) if q_in is not None else ActLayout(0, 0, 0, 0, 0)
@@ -567,7 +576,7 @@ def kv_write(q_in, q_out, k_new, v_new, start_pos, n_new, kv: KvLayout, q_gain=N
 
 @_on_device_of(0)
 def selftest_umma(a: torch.Tensor, b: torch.Tensor):
-    lib = init(a.device.index)
+    lib = init(a.get_device())
     out = torch.zeros(4, 128, 128, dtype=torch.float32, device=a.device)
     status = torch.full((4,), -1, dtype=torch.int32, device=a.device)
     _check(lib.kb200_selftest_umma(_ptr(a), _ptr(b), _ptr(out), _ptr(status), _stream()), "kb200_selftest_umma")
@@ -579,7 +588,7 @@ def selftest_wait_timeout(device, limit_ns: int = 1_000_000, code: int = 77) -> 
     The device status word then holds `code` until read_status() / check_status() clears it."""
     result = torch.zeros(3, dtype=torch.int32, device=device)
     with torch.cuda.device(result.device):
-        lib = init(result.device.index)
+        lib = init(result.get_device())
         _check(lib.kb200_selftest_wait_timeout(_ptr(result), int(limit_ns), int(code), _stream()),
                "kb200_selftest_wait_timeout")
     _launched(1)

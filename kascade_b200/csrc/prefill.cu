@@ -1406,7 +1406,7 @@ extern "C" int kb200_read_status(int* host_out) {
   KB_REQUIRE(host_out, "read_status: null pointer");
   int zero = 0;
   KB_CUDA(cudaMemcpyFromSymbol(host_out, g_status_word, sizeof(int)));
-  KB_CUDA(cudaMemcpyToSymbol(g_status_word, &zero, sizeof(int)));
+  if (*host_out != 0) KB_CUDA(cudaMemcpyToSymbol(g_status_word, &zero, sizeof(int)));   // a second round trip only if set
   return 0;
 }
 

@@ -159,6 +159,7 @@ class EfficientKascadeStrategy(Strategy):
         self._dec_kmax = 0
         self._map_dev: Dict[tuple, torch.Tensor] = {}
         self._buf: Dict[str, torch.Tensor] = {}
+        self._views: Dict[str, tuple] = {}
         super().__init__("efficient_kascade")
 
     # ------------------------------------------------------------------------------------------
@@ -208,13 +209,19 @@ class EfficientKascadeStrategy(Strategy):
 
     # ------------------------------------------------------------------------------------------
     def _scratch(self, name: str, shape, dtype, device) -> torch.Tensor:
-        """Grow-only cache of device buffers, so steady-state calls allocate nothing."""
+        """Grow-only cache of device buffers, so steady-state calls allocate nothing; the view of the last shape is kept
+        with the buffer, since the layers of a step ask for the same one."""
+        last = self._views.get(name)
+        if last is not None and last[0] == shape and last[1] == dtype and last[2] == device:
+            return last[3]
         n = int(math.prod(shape))
         buf = self._buf.get(name)
         if buf is None or buf.numel() < n or buf.dtype != dtype or buf.device != device:
             buf = torch.empty(max(n, 1), dtype=dtype, device=device)
             self._buf[name] = buf
-        return buf[:n].view(*shape)
+        view = buf[:n].view(*shape)
+        self._views[name] = (shape, dtype, device, view)
+        return view
 
     def _mapping(self, layer_idx: int, device) -> torch.Tensor:
         key = (layer_idx, device)
@@ -231,7 +238,8 @@ class EfficientKascadeStrategy(Strategy):
     def _token_major(x: torch.Tensor) -> torch.Tensor:
         """[B, heads, L, D] -> a [B, L, heads, D] view with D contiguous and 16-byte aligned strides."""
         y = x.transpose(1, 2)
-        if y.stride(3) != 1 or any(s % 8 for s in y.stride()[:3]) or y.data_ptr() % 16:
+        b, t, h, d = y.stride()
+        if d != 1 or b % 8 or t % 8 or h % 8 or y.data_ptr() % 16:
             y = y.contiguous()
         return y
 
@@ -255,16 +263,14 @@ class EfficientKascadeStrategy(Strategy):
                 return self._decode_padded(pad, module, query, key, value, scaling), None
             if Lq != Lk:
                 raise NotImplementedError("prefill expects the whole prompt (Lq == Lk); chunked prefill is not supported")
-            starts, lens = pad
-            dev = query.device
-            rg = (torch.tensor(starts, dtype=torch.int32, device=dev), torch.tensor(lens, dtype=torch.int32, device=dev), lens)
             q, k, v = self._token_major(query), self._token_major(key), self._token_major(value)
-            return self._prefill(layer, q, k, v, scaling, ragged=rg), None
+            return self._prefill(layer, q, k, v, scaling, ragged=self._pad_bounds(pad, query.device)), None
         if Lq == 1:
             kv = nat.kv_layout_contiguous(*self._cache_views(key, value))
-            seq_lens = self._scratch("seq_lens_full", (B,), torch.int32, query.device)
-            seq_lens.fill_(Lk)
             dense = Lk <= 128                      # strategies/EfficientKascadeStrategy.py:137-140
+            seq_lens = self._scratch("seq_lens_full", (B,), torch.int32, query.device)
+            if dense or self.is_anchor(layer):     # a reuse layer's kernels read the counts of the index rows instead
+                seq_lens.fill_(Lk)
             out = self._decode(layer, query[:, :, 0], kv, seq_lens, Lk, scaling, G, dense_only=dense)
             return out.unsqueeze(1), None
         if Lq != Lk:
@@ -304,6 +310,15 @@ class EfficientKascadeStrategy(Strategy):
             self._pads = None if all(n == Lk for n in lens) else (starts, lens)
         return self._pads
 
+    def _pad_bounds(self, pad, dev):
+        """(first rows, lengths) of a padded batch on the device and its lengths on the host; copied once per mask, not
+        once per layer."""
+        cached = getattr(self, "_pad_dev", None)
+        if cached is None or cached[0] is not pad or cached[1].device != dev:
+            both = torch.tensor(pad, dtype=torch.int32, device=dev)
+            cached = self._pad_dev = (pad, both[0], both[1], pad[1])
+        return cached[1:]
+
     def _decode_padded(self, pad, module, query, key, value, scaling) -> torch.Tensor:
         """One decode step of a padded batch, every kernel launched once: the cache rows of sequence b are
         starts[b] .. starts[b] + lens[b] - 1, described to the decode kernels as a block table with one-token pages
@@ -329,7 +344,8 @@ class EfficientKascadeStrategy(Strategy):
 
     @staticmethod
     def _cache_views(key, value):
-        if key.stride(3) != 1 or any(s % 8 for s in key.stride()[:3]) or key.stride() != value.stride():
+        b, h, t, d = st = key.stride()
+        if d != 1 or b % 8 or h % 8 or t % 8 or st != value.stride():
             key, value = key.contiguous(), value.contiguous()
         return key, value
 
@@ -488,9 +504,9 @@ class EfficientKascadeStrategy(Strategy):
         longest sequence is `raggedness` times the mean the CTAs of the long ones would set the kernel's time, so
         they are cut until the longest CTA is about the batch's work divided by three CTAs per SM (measured on
         batches of 32-128 sequences of 4k-65k tokens: 10-19 % faster at 32 and 64 sequences, no change at 128)."""
-        s = nat.decode_default_splits(B, G, keys_max)
+        s = nat.decode_default_splits(B, G, keys_max, dev.index)
         if raggedness > 1.25:
-            slots = 3 * torch.cuda.get_device_properties(dev).multi_processor_count
+            slots = 3 * nat.sm_count(dev.index)
             want = -(-int(raggedness * slots) // max(B * G, 1))
             s = max(s, min(want, max(keys_max // 256, 1), 32))
         return s
