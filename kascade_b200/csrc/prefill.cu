@@ -25,15 +25,17 @@
 //   with V, sparse (512 threads): warps 8-10 gather the selected K rows and warps 11, 14, 15 the V rows
 //     with cp.async (16-byte chunks, 16 lanes per 256-byte row, written directly in the
 //     128-byte-swizzled operand layout of umma.cuh); warp 12 issues Q.K^T, warp 13 P.V.
-//   without V (640 threads):      warps 0-15 four softmax / reducer warpgroups (key block n of the CTA belongs
-//     to warpgroup n mod 4); warp 16 lane 0 TMA copies, warp 17 issues Q.K^T.
+//   lse only (512 threads):       warps 0-11 three softmax warpgroups (key blocks j = w mod 3); warp 12 lane 0 TMA
+//     copies, warp 13 issues Q.K^T.
+//   pool (640 threads):           warps 0-15 four reducer warpgroups (key block n of the CTA belongs to warpgroup
+//     n mod 4); warp 16 lane 0 TMA copies, warp 17 issues Q.K^T.
 // setmaxnreg moves registers from the producer / MMA warpgroups to the softmax warpgroups.
 // Hand-offs are mbarriers; every wait is bounded (umma::mbar_wait) and a kernel that gives up
 // records a code in the device status word, drains its copies, frees its tensor memory and returns.
 //
 // Tensor memory (512 columns).  With V: S0 [0,128), S1 [128,256), P0 [256,320), P1 [320,384) (fp16 pairs,
 // the A operand of P.V), O [384,512) - one accumulator for both streams, see the softmax role.
-// Without V: S0, S1, S2, S3.
+// Without V: S0, S1, S2 (and S3, pool).
 #include <cuda.h>
 #include <stdlib.h>
 
@@ -149,17 +151,11 @@ __device__ __forceinline__ uint64_t ex2_fma2(uint64_t x2) {
   unpair_f(t, t0, t1);
   return pair_u(__float_as_uint(q0) + (__float_as_uint(t0) << 23), __float_as_uint(q1) + (__float_as_uint(t1) << 23));
 }
-// 2^x of pair number `pair` (0..15) of 32 values: kPolyShare of the 16 pairs, evenly spread, go to the FMA pipes.  The
-// two-element fma occupies the heavy FMA pipe for two cycles, so that pipe (256 + 56 * share cycles per block) and
-// the special-function unit (1024 - 64 * share) meet at a share of 5-6.  Measured with four streams at 8192 tokens,
-// share 0 / 3 / 4 / 5 / 6 / 16: pool 364 / 313 / 301 / 292 / 295 / 481 us, lse 361 / 325 / 326 / 331 / 333 / 494 us.
-constexpr int kPolyShare = 5;
-__device__ __forceinline__ uint64_t ex2_pair(int pair, uint64_t x) {
-  if (((pair + 1) * kPolyShare >> 4) != (pair * kPolyShare >> 4)) return ex2_fma2(x);
-  float x0, x1;
-  unpair_f(x, x0, x1);
-  return pair_f(ex2(x0), ex2(x1));
-}
+// Which exponentials take that way: of every eight values the fourth and eighth in the lse pass, and the second as
+// well in the pool pass.  The two-element fma occupies the heavy FMA pipe for two cycles, so that pipe (256 + 56 s
+// cycles per block with s of 16 values) and the special-function unit (1024 - 64 s) meet at s = 5-6.  Measured at
+// 8192 tokens, s = 0 / 3 / 4 / 5 / 6 / 16: pool 364 / 313 / 301 / 292 / 295 / 481 us, lse 361 / 325 / 326 / 331 / 333 /
+// 494 us.  The choice is part of the scores' last bits, and so of which of two equal keys is selected.
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;\n" : "=f"(d) : "f"(a), "f"(b), "f"(c));
@@ -196,8 +192,7 @@ struct PfShared {
 static_assert(sizeof(PfShared) <= 2560, "PfShared grew");
 constexpr int kSmemAttn = kStageBytes * (1 + 3 + kNV) + kPadAllowance + 2560;   // = 232448, the sm_100 limit
 constexpr int kNQNoV = 2, kNKNoV = 4;         // Q tiles and K ring of the modes without V
-constexpr int kStreamsNoV = 4;
-constexpr int kXchgNoV = kStreamsNoV * 2 * 128 * 4;   // their exchange area behind PfShared: two values per stream and row
+constexpr int kXchgNoV = 4 * 2 * 128 * 4;   // their exchange area behind PfShared: two values per stream and row
 constexpr int kSmemNoV = kStageBytes * (kNQNoV + kNKNoV) + kPadAllowance + 2560 + kXchgNoV;
 
 // One work item = one query tile of one KV head of one sequence.
@@ -251,18 +246,18 @@ struct PfCfg {
   static constexpr bool kHasV = MODE == kDenseAttn || MODE == kSparse;
   static constexpr bool kIsPool = MODE == kPool;
   static constexpr bool kGather = MODE == kSparse;
-  // softmax warpgroups (streams): two with V; four without, where a block has no accumulator and no probabilities
-  // to keep and a thread holds half a row at a time (104 registers).  Against three streams that hold whole rows, at
-  // 16384 tokens: lse 1405 -> 1285 us, pool 1345 -> 1190 us, together with the issuer's early look and the second Q tile.
-  static constexpr int kStreams = kHasV ? 2 : kStreamsNoV;
+  // softmax warpgroups (streams): two with V; three in the lse mode, whose threads hold whole rows; four in the pool
+  // mode, where a thread needs no more than half of a row at a time (104 registers): against three, at 16384 tokens,
+  // 1270 -> 1222 us (lse 1286 -> 1267: not worth the other grouping of its partial sums).
+  static constexpr int kStreams = kHasV ? 2 : kIsPool ? 4 : 3;
   static constexpr int kSoftmaxWarps = 4 * kStreams;
-  static constexpr int kThreads = !kHasV ? 640 : kGather ? 512 : 384;
+  static constexpr int kThreads = kIsPool ? 640 : (kGather || !kHasV) ? 512 : 384;
   static constexpr int kNQ = kHasV ? 1 : kNQNoV;
   static constexpr int kNK = kHasV ? 3 : kNKNoV;
   static constexpr int kProducerArrivals = 1;                   // Q tile: one thread announces the TMA bytes
   static constexpr int kRingArrivals = kGather ? 96 : 1;        // K / V stage: three gather warps each
-  static constexpr int kProducerWarp0 = kHasV ? 8 : 16;
-  static constexpr int kMmaWarp = kGather ? 12 : (kHasV ? 9 : 17);
+  static constexpr int kProducerWarp0 = kHasV ? 8 : kSoftmaxWarps;
+  static constexpr int kMmaWarp = kGather ? 12 : (kHasV ? 9 : kSoftmaxWarps + 1);
 };
 
 template <int MODE, bool BF16>
@@ -293,7 +288,7 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
   if (tid == 0) sh.abort = *reinterpret_cast<volatile int*>(&g_status_word);
   __syncthreads();
   if (sh.abort != 0) return;
-  // modes without V: [4 streams][2][128] floats behind PfShared (partial row statistics / staged lse values)
+  // modes without V: [streams][2][128] floats behind PfShared (partial row statistics / staged lse values)
   float* const xchg_nov = reinterpret_cast<float*>(smem + kTiles * kStageBytes + 2560);
   uint64_t* bar_kfull = sh.bar_kfull;
   uint64_t* bar_kempty = sh.bar_kempty;
@@ -498,8 +493,9 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
   };
 
   // ================================ MMA issuer, modes without V ===================================
-  // The key blocks of a CTA are numbered n = 0, 1, 2, ... across all its tiles; block n goes through S buffer
-  // n % kStreams and K stage n % kNK.  The tensor core holds only a few products in its queue, so an issuer that
+  // The key blocks of a CTA are numbered n = 0, 1, 2, ... across all its tiles; block n goes through K stage n % kNK
+  // and, in the pool mode, S buffer n % kStreams (in the lse mode block j of a tile through buffer j % kStreams: which
+  // blocks are summed together then depends on the tile alone).  The tensor core holds only a few products in its queue, so an issuer that
   // starts its waits for block n + 1 after block n's products leaves it idle between blocks: it looks at block
   // n + 1's barriers before the last product of block n, and waits only if they were not complete by then.  With
   // the softmax work left out, this and the second Q tile took the pass from 254 to 191 us at 8192 tokens (the
@@ -507,7 +503,16 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
   auto mma_role = [&]() {
     constexpr uint32_t idesc_qk = idesc_f16(128, 128, 0, 0, BF16);
     constexpr int NS = Cfg::kStreams;
-    int n = 0, qn = 0;
+    int n = 0, qn = 0, w = 0;                           // blocks and Q tiles so far, S buffer of block n
+    int used[NS];                                       // blocks issued into each S buffer so far
+#pragma unroll
+    for (int i = 0; i < NS; ++i) used[i] = 0;
+    auto used_of = [&](int b) {
+      int u = used[0];
+#pragma unroll
+      for (int i = 1; i < NS; ++i) u = b == i ? used[i] : u;
+      return u;
+    };
     bool ok = true, have = false;                       // have: block n's barriers have been seen complete
     // the whole warp runs this role with uniform control flow; one elected lane issues
     const bool el = elect_one();
@@ -523,10 +528,11 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
       ++qn;
       const uint32_t q_lo = q_lo0 + qb * (kStageBytes >> 4);
       for (int j = 0; j < it.nb; ++j) {
-        const int w = n % NS, st = n % kNK;
+        const int st = n % kNK;
         if (!have) {
           // S buffer w may be overwritten once the block issued into it before has been consumed
-          if (n >= NS) ok = mbar_wait(&bar_pready[w], (n / NS - 1) & 1, &give_up, 23);
+          const int u = used_of(w);
+          if (u > 0) ok = mbar_wait(&bar_pready[w], (u - 1) & 1, &give_up, 23);
           if (ok) ok = mbar_wait(&bar_kfull[st], (n / kNK) & 1, &give_up, 22);
           if (!ok) break;
         }
@@ -542,14 +548,19 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
 #pragma unroll
           for (int ks = 0; ks < 7; ++ks) issue(ks);
         }
+        const int w_now = w;
+#pragma unroll
+        for (int i = 0; i < NS; ++i) used[i] += i == w;
+        w = w + 1 == NS || (!POOL && j + 1 == it.nb) ? 0 : w + 1;
         ++n;
-        have = (n < NS || mbar_test_wait(&bar_pready[n % NS], (n / NS - 1) & 1)) &&
+        const int u_next = used_of(w);
+        have = (u_next == 0 || mbar_test_wait(&bar_pready[w], (u_next - 1) & 1)) &&
                mbar_test_wait(&bar_kfull[n % kNK], (n / kNK) & 1);
         have = __all_sync(0xFFFFFFFFu, have);           // the lanes may have looked at different moments
         if (el) {
           issue(7);
           mma_commit(&bar_kempty[st]);
-          mma_commit(&bar_sfull[w]);
+          mma_commit(&bar_sfull[w_now]);
           if (j + 1 == it.nb) mma_commit(&sh.bar_qempty[qb]);   // the tile's last product is queued
         }
         __syncwarp();
@@ -958,11 +969,11 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
   };
 
   // ================================ softmax statistics only (no V) ================================
-  // Four warpgroups, four independent streams: warpgroup w owns the key blocks n = w mod 4 of the CTA with its own S
-  // buffer and its own running (max, sum) per row, so the tcgen05.ld / max / ex2 phases of one stream overlap
-  // those of the others and nothing is exchanged per block.  A thread reads its row from tensor memory in halves of
-  // 64 values (the lower half twice), which is what lets four streams fit the register file.  The partial results
-  // of a row are merged like split-K partials in the epilogue.
+  // Three warpgroups, three independent streams: warpgroup w owns the key blocks j = w, w+3, ... of
+  // every tile with its own S buffer and its own running (max, sum) per row, so the tcgen05.ld / max /
+  // ex2 phases of one stream overlap those of the others and nothing is exchanged per block (with two
+  // streams no unit was busy more than 64 %: three warps per SM sub-partition hide each other's
+  // latencies better).  The partial results of a row are merged like split-K partials in the epilogue.
   auto softmax_role = [&]() {
     const int wg = warp >> 2;
     const int row = (warp & 3) * 32 + lane, q_local = row >> 2;
@@ -971,7 +982,7 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
     constexpr int NS = Cfg::kStreams;
     float* const xm = xchg_nov;                           // [NS][128] partial maxima
     float* const xl = xchg_nov + NS * 128;                // [NS][128] partial sums
-    int n0 = 0, tiles_done = 0;                        // blocks of the tiles before this one, tiles finished
+    int done_mine = 0, tiles_done = 0;                 // blocks finished by this stream, tiles finished
     bool ok = true;
     for (int k = 0; k < n_rounds && ok; ++k) {
       const int item = item_of(k);
@@ -980,40 +991,39 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
       if (it.nb == 0) continue;
       const int tok = it.tile_start + q_local;
       const int off = it.tile_start;                    // slot - off = key position inside the tile
+      const int n_mine = it.nb > wg ? (it.nb - wg + NS - 1) / NS : 0;
       float m_run = -INFINITY, l_run = 0.f;             // m_run in the scaled (log2) domain
-      for (int j = (wg + NS - n0 % NS) % NS; j < it.nb; j += NS) {
-        ok = mbar_wait(&bar_sfull[wg], ((n0 + j) / NS) & 1, &give_up, 31);
+      for (int j = wg, jj = 0; j < it.nb; j += NS, ++jj) {
+        ok = mbar_wait(&bar_sfull[wg], (done_mine + jj) & 1, &give_up, 31);
         if (!ok) break;
         tc_fence_after();
         const int c0 = j * 128 - off;                     // key position (inside the tile) of column 0
         const bool need_mask = (c0 + 127) > 0;            // only the last block(s) of a tile
-        uint32_t sa[32], sb[32];
-        auto load_half = [&](int c) {
-          tmem_ld32(ts + c, sa);
-          tmem_ld32(ts + c + 32, sb);
-          tmem_wait_ld();
-          if (need_mask) {
+        // the whole S row (128 fp32) comes into registers with one round trip to tensor memory
+        uint32_t sr[4][32];
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              if ((c0 + c + i) > q_local) sa[i] = 0xFF800000u;     // -inf
-              if ((c0 + c + 32 + i) > q_local) sb[i] = 0xFF800000u;
-            }
-          }
-        };
+        for (int part = 0; part < 4; ++part) tmem_ld32(ts + part * 32, sr[part]);
+        tmem_wait_ld();
+        tc_fence_before();
+        mbar_arrive(&bar_pready[wg]);                     // S is in registers: the buffer may be refilled
+        if (need_mask) {
+#pragma unroll
+          for (int part = 0; part < 4; ++part)
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if ((c0 + part * 32 + i) > q_local) sr[part][i] = 0xFF800000u;     // -inf
+        }
         float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
-        auto max_half = [&]() {
 #pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            mx0 = max3(mx0, __uint_as_float(sa[i]), __uint_as_float(sa[i + 1]));
-            mx1 = max3(mx1, __uint_as_float(sa[i + 2]), __uint_as_float(sa[i + 3]));
-            mx2 = max3(mx2, __uint_as_float(sb[i]), __uint_as_float(sb[i + 1]));
-            mx3 = max3(mx3, __uint_as_float(sb[i + 2]), __uint_as_float(sb[i + 3]));
+        for (int part = 0; part < 4; ++part) {
+#pragma unroll
+          for (int i = 0; i < 32; i += 8) {
+            mx0 = max3(mx0, __uint_as_float(sr[part][i]), __uint_as_float(sr[part][i + 1]));
+            mx1 = max3(mx1, __uint_as_float(sr[part][i + 2]), __uint_as_float(sr[part][i + 3]));
+            mx2 = max3(mx2, __uint_as_float(sr[part][i + 4]), __uint_as_float(sr[part][i + 5]));
+            mx3 = max3(mx3, __uint_as_float(sr[part][i + 6]), __uint_as_float(sr[part][i + 7]));
           }
-        };
-        load_half(0);
-        max_half();
-        load_half(64);
-        max_half();
+        }
         const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * p.scale2;
         // The reference point of the exponentials only moves when the row maximum has grown by more
         // than 2^kRescaleLog2 (the terms then stay below 2^kRescaleLog2, exact in fp32);
@@ -1022,20 +1032,23 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
         const float alpha = ex2(m_run - m_new);
         uint64_t s01 = 0ull, s23 = 0ull;                    // four partial row sums, two per register pair
         const uint64_t scale_2 = pair_f(p.scale2, p.scale2), nref_2 = pair_f(-m_new, -m_new);
-        auto sum_part = [&](const uint32_t (&sr)[32]) {
 #pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            s01 = add2(s01, ex2_pair(i >> 1, fma2(pair_u(sr[i], sr[i + 1]), scale_2, nref_2)));
-            s23 = add2(s23, ex2_pair((i >> 1) + 1, fma2(pair_u(sr[i + 2], sr[i + 3]), scale_2, nref_2)));
+        for (int part = 0; part < 4; ++part)
+#pragma unroll
+          for (int i = 0; i < 32; i += 8) {
+            float x[8], e[8];
+#pragma unroll
+            for (int k2 = 0; k2 < 8; k2 += 2)
+              unpair_f(fma2(pair_u(sr[part][i + k2], sr[part][i + k2 + 1]), scale_2, nref_2), x[k2], x[k2 + 1]);
+            unpair_f(ex2_fma2(pair_f(x[3], x[7])), e[3], e[7]);
+            e[0] = ex2(x[0]); e[1] = ex2(x[1]); e[2] = ex2(x[2]);
+            e[4] = ex2(x[4]); e[5] = ex2(x[5]); e[6] = ex2(x[6]);
+#pragma unroll
+            for (int k2 = 0; k2 < 8; k2 += 4) {
+              s01 = add2(s01, pair_f(e[k2], e[k2 + 1]));
+              s23 = add2(s23, pair_f(e[k2 + 2], e[k2 + 3]));
+            }
           }
-        };
-        sum_part(sa);
-        sum_part(sb);
-        load_half(0);
-        tc_fence_before();
-        mbar_arrive(&bar_pready[wg]);                     // S has been read for the last time: the buffer may be refilled
-        sum_part(sa);
-        sum_part(sb);
         float s0, s1, s2, s3;
         unpair_f(s01, s0, s1);
         unpair_f(s23, s2, s3);
@@ -1043,7 +1056,7 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
         m_run = m_new;
       }
       if (!ok) break;
-      n0 += it.nb;
+      done_mine += n_mine;
       // ---- epilogue: merge the streams, store ------------------------------------------------
       // the exchange buffer is free once both warpgroups have finished the previous tile's epilogue
       if (tiles_done > 0) {
@@ -1111,11 +1124,26 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
         const uint64_t scale_2 = pair_f(p.scale2, p.scale2);
         auto sum_part = [&](const uint32_t (&sr)[32], int part) {
 #pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            // the four rows' lse2 with one 16-byte shared-memory load (the same address for the whole warp)
-            const float4 l4 = reinterpret_cast<const float4*>(lse_s)[part * 8 + (i >> 2)];   // holds -lse2
-            a01 = add2(a01, ex2_pair(i >> 1, fma2(pair_u(sr[i], sr[i + 1]), scale_2, pair_f(l4.x, l4.y))));
-            a23 = add2(a23, ex2_pair((i >> 1) + 1, fma2(pair_u(sr[i + 2], sr[i + 3]), scale_2, pair_f(l4.z, l4.w))));
+          for (int i = 0; i < 32; i += 16) {
+            float x[16], e[16];
+#pragma unroll
+            for (int k2 = 0; k2 < 16; k2 += 4) {
+              // the four rows' lse2 with one 16-byte shared-memory load (the same address for the whole warp)
+              const float4 l4 = reinterpret_cast<const float4*>(lse_s)[part * 8 + ((i + k2) >> 2)];   // holds -lse2
+              unpair_f(fma2(pair_u(sr[i + k2], sr[i + k2 + 1]), scale_2, pair_f(l4.x, l4.y)), x[k2], x[k2 + 1]);
+              unpair_f(fma2(pair_u(sr[i + k2 + 2], sr[i + k2 + 3]), scale_2, pair_f(l4.z, l4.w)), x[k2 + 2], x[k2 + 3]);
+            }
+            unpair_f(ex2_fma2(pair_f(x[1], x[3])), e[1], e[3]);
+            unpair_f(ex2_fma2(pair_f(x[7], x[9])), e[7], e[9]);
+            unpair_f(ex2_fma2(pair_f(x[11], x[15])), e[11], e[15]);
+#pragma unroll
+            for (int k2 = 0; k2 < 16; ++k2)
+              if (k2 != 1 && k2 != 3 && k2 != 7 && k2 != 9 && k2 != 11 && k2 != 15) e[k2] = ex2(x[k2]);
+#pragma unroll
+            for (int k2 = 0; k2 < 16; k2 += 4) {
+              a01 = add2(a01, pair_f(e[k2], e[k2 + 1]));
+              a23 = add2(a23, pair_f(e[k2 + 2], e[k2 + 3]));
+            }
           }
         };
         uint32_t sa[32], sb[32];                            // 64 of the 128 values at a time, the next part on its way
@@ -1151,12 +1179,15 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
   // The instruction is warpgroup-wide: all four warps of a warpgroup execute the same one, and the role
   // code sits inside the branch that issued it.
   if (!HAS_V) {
-    //   no V : 640 threads x 96 at launch; 512 x 104 + 128 x 64 = 61440 = 640 x 96; 4 x 104 + 64 = 480
+    //   lse  : 512 threads x 128 at launch; 384 x 152 + 128 x 56 = 65536; 3 x 152 + 56 = 512
+    //   pool : 640 threads x 96 at launch; 512 x 104 + 128 x 64 = 61440 = 640 x 96; 4 x 104 + 64 = 480
     if (warp < Cfg::kSoftmaxWarps) {
-      asm volatile("setmaxnreg.inc.sync.aligned.u32 104;\n");
+      if (POOL) asm volatile("setmaxnreg.inc.sync.aligned.u32 104;\n");
+      else asm volatile("setmaxnreg.inc.sync.aligned.u32 152;\n");
       if (POOL) pool_role(); else softmax_role();
     } else {
-      asm volatile("setmaxnreg.dec.sync.aligned.u32 64;\n");
+      if (POOL) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;\n");
+      else asm volatile("setmaxnreg.dec.sync.aligned.u32 56;\n");
       if (warp == Cfg::kProducerWarp0) {
         if (lane == 0) producer_tma();
         __syncwarp();

@@ -236,3 +236,35 @@ def test_rejected_arguments_name_the_problem():
     with pytest.raises(nat.KascadeNativeError, match="power of two"):
         nat.kv_write(None, None, k, k, torch.zeros(B, dtype=torch.int32, device=dev), None, nat.kv_layout_paged(kc, kc, bt))
     assert nat.read_status() == 0
+
+
+@pytest.mark.parametrize("L", [1, 31, 33, 128, 129, 160, 385, 513, 640, 1025])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_lse_and_pooled_scores_at_the_edges_of_the_streams(L, dtype):
+    """The passes without V deal key blocks of 128 to three (lse) and four (pool) streams and keep two Q tiles: prompts of
+    1 to 9 blocks, full and ragged last blocks, against 64 bits.  Products are exact in fp32, a row's 128 to 1025 terms and
+    their polynomial exponentials (3e-6) add up to well under 2e-5; pooled scores are sums of such terms."""
+    from kascade_b200 import _native as nat
+    dev = torch.device("cuda")
+    g = torch.Generator().manual_seed(L)
+    B, H, G, D, tile = 2, 8, 2, 128, 32
+    q = torch.randn(B, L, H, D, generator=g).to(dtype).to(dev)
+    k = torch.randn(B, L, G, D, generator=g).to(dtype).to(dev)
+    T, scale = -(-L // tile), 0.6 * D ** -0.5
+    lse2 = torch.empty(B, L, H, dtype=torch.float32, device=dev)
+    pooled = torch.full((B, G, T, -(-L // 128) * 128), -7.0, device=dev)
+    nat.prefill_dense(q, k, None, scale, None, lse2)
+    nat.prefill_pool_scores(q, k, lse2, scale, pooled)
+    s = torch.einsum("bighd,bjgd->bghij", q.double().view(B, L, G, 4, D), k.double()) * scale
+    s = s.masked_fill(~torch.ones(L, L, dtype=torch.bool, device=dev).tril(), float("-inf"))
+    want = torch.logsumexp(s, -1)
+    got = lse2.double().view(B, L, G, 4).permute(0, 2, 3, 1) * 0.6931471805599453
+    assert (got - want).abs().max().item() < 2e-5
+    p = torch.softmax(s, -1).sum(2)                                   # [B, G, i, j]
+    for t in range(T):
+        start = t * tile
+        ref = p[:, :, start:start + tile, :start].sum(2)
+        if start:
+            assert ((pooled[:, :, t, :start].double() - ref).abs() / ref.clamp_min(1e-6)).max().item() < 5e-5, t
+        assert bool((pooled[:, :, t, start:] == -7.0).all()), "entries from the tile on are not written"
+    assert nat.read_status() == 0
