@@ -52,6 +52,34 @@ constexpr int kHg = KB200_GROUP_SIZE;    // query heads per KV head
 constexpr int kTile = KB200_TILE;        // queries per prefill tile
 constexpr float kLog2e = 1.4426950408889634f;
 
+// Programmatic dependent launch.  Every kernel of the attention path starts with pdl_begin(): it waits until the kernel
+// before it in the stream has completed and its writes are visible, then lets the kernel after it be set up.  That
+// one's launch, block scheduling and parameter loads so fall into this one's run time instead of a gap of 1.5-2 us
+// after it.  Nothing may touch global memory before the wait.
+__device__ __forceinline__ void pdl_begin() {
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+// launches a kernel that begins with pdl_begin(), as a cluster of `cluster` CTAs along x if that is not 1
+template <typename... P, typename... A>
+static inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st,
+                                     unsigned cluster, const A&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 __host__ __device__ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 int sm_count();

@@ -272,6 +272,7 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
   constexpr int kNK = Cfg::kNK;
   constexpr int kMmaWarp = Cfg::kMmaWarp;
 
+  pdl_begin();
   extern __shared__ uint8_t smem_raw[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t pad = (1024u - (smem_addr(smem_raw) & 1023u)) & 1023u;
@@ -1497,15 +1498,16 @@ static int prefill_dense_impl(const kb200_act_layout* q, const kb200_act_layout*
   if (out && make_act_map(&tv, p.v, p.v_sb, p.v_st, p.v_sh, num_kv_heads, seq_len, batch, 1, 128, "v") != 0) return -1;
   dim3 grid(persistent_grid(p));
   if (same_dtype(&p, q, k, out ? v : nullptr, "prefill_dense") != 0) return -1;
+  cudaError_t rc;
   if (out && p.bf16)
-    tile_prefill_kernel<kDenseAttn, true><<<grid, PfCfg<kDenseAttn>::kThreads, kSmemAttn, (cudaStream_t)stream>>>(p, tq, tk, tv);
+    rc = launch_pdl(tile_prefill_kernel<kDenseAttn, true>, grid, PfCfg<kDenseAttn>::kThreads, kSmemAttn, (cudaStream_t)stream, 1, p, tq, tk, tv);
   else if (out)
-    tile_prefill_kernel<kDenseAttn, false><<<grid, PfCfg<kDenseAttn>::kThreads, kSmemAttn, (cudaStream_t)stream>>>(p, tq, tk, tv);
+    rc = launch_pdl(tile_prefill_kernel<kDenseAttn, false>, grid, PfCfg<kDenseAttn>::kThreads, kSmemAttn, (cudaStream_t)stream, 1, p, tq, tk, tv);
   else if (p.bf16)
-    tile_prefill_kernel<kDenseLse, true><<<grid, PfCfg<kDenseLse>::kThreads, kSmemNoV, (cudaStream_t)stream>>>(p, tq, tk, tv);
+    rc = launch_pdl(tile_prefill_kernel<kDenseLse, true>, grid, PfCfg<kDenseLse>::kThreads, kSmemNoV, (cudaStream_t)stream, 1, p, tq, tk, tv);
   else
-    tile_prefill_kernel<kDenseLse, false><<<grid, PfCfg<kDenseLse>::kThreads, kSmemNoV, (cudaStream_t)stream>>>(p, tq, tk, tv);
-  KB_CHECK_LAUNCH("tile_prefill_kernel<dense>");
+    rc = launch_pdl(tile_prefill_kernel<kDenseLse, false>, grid, PfCfg<kDenseLse>::kThreads, kSmemNoV, (cudaStream_t)stream, 1, p, tq, tk, tv);
+  KB_CUDA(rc);
   return 0;
 }
 }  // namespace kb200
@@ -1551,11 +1553,12 @@ static int prefill_pool_impl(const kb200_act_layout* q, const kb200_act_layout* 
   if (make_act_map(&tk, p.k, p.k_sb, p.k_st, p.k_sh, num_kv_heads, seq_len, batch, 1, 128, "k") != 0) return -1;
   dim3 grid(persistent_grid(p));
   if (same_dtype(&p, q, k, nullptr, "prefill_pool_scores") != 0) return -1;
+  cudaError_t rc;
   if (p.bf16)
-    tile_prefill_kernel<kPool, true><<<grid, PfCfg<kPool>::kThreads, kSmemNoV, (cudaStream_t)stream>>>(p, tq, tk, tk);
+    rc = launch_pdl(tile_prefill_kernel<kPool, true>, grid, PfCfg<kPool>::kThreads, kSmemNoV, (cudaStream_t)stream, 1, p, tq, tk, tk);
   else
-    tile_prefill_kernel<kPool, false><<<grid, PfCfg<kPool>::kThreads, kSmemNoV, (cudaStream_t)stream>>>(p, tq, tk, tk);
-  KB_CHECK_LAUNCH("tile_prefill_kernel<pool>");
+    rc = launch_pdl(tile_prefill_kernel<kPool, false>, grid, PfCfg<kPool>::kThreads, kSmemNoV, (cudaStream_t)stream, 1, p, tq, tk, tk);
+  KB_CUDA(rc);
   return 0;
 }
 }  // namespace kb200
@@ -1623,11 +1626,12 @@ static int prefill_sparse_impl(const kb200_act_layout* q, const kb200_act_layout
   if (make_act_map(&tq, p.q, p.q_sb, p.q_st, p.q_sh, num_q_heads, seq_len, batch, kHg, kTile, "q") != 0) return -1;
   dim3 grid(persistent_grid(p));
   if (same_dtype(&p, q, k, v, "prefill_sparse") != 0) return -1;
+  cudaError_t rc;
   if (p.bf16)
-    tile_prefill_kernel<kSparse, true><<<grid, PfCfg<kSparse>::kThreads, kSmemAttn, (cudaStream_t)stream>>>(p, tq, none, none);
+    rc = launch_pdl(tile_prefill_kernel<kSparse, true>, grid, PfCfg<kSparse>::kThreads, kSmemAttn, (cudaStream_t)stream, 1, p, tq, none, none);
   else
-    tile_prefill_kernel<kSparse, false><<<grid, PfCfg<kSparse>::kThreads, kSmemAttn, (cudaStream_t)stream>>>(p, tq, none, none);
-  KB_CHECK_LAUNCH("tile_prefill_kernel<sparse>");
+    rc = launch_pdl(tile_prefill_kernel<kSparse, false>, grid, PfCfg<kSparse>::kThreads, kSmemAttn, (cudaStream_t)stream, 1, p, tq, none, none);
+  KB_CUDA(rc);
   return 0;
 }
 }  // namespace kb200

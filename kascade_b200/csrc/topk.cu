@@ -164,6 +164,7 @@ topk_select_kernel(const float* __restrict__ scores, int64_t row_stride, int n_c
   extern __shared__ uint32_t merged[];                    // C > 1: the lists of all CTAs of the cluster
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rank = C > 1 ? (int)cg::this_cluster().block_rank() : 0;
+  pdl_begin();
 
   for (int64_t row = blockIdx.x / C; row < rows; row += gridDim.x / C) {
     int n, k;
@@ -613,6 +614,7 @@ topk_select_kernel(const float* __restrict__ scores, int64_t row_stride, int n_c
 
 __global__ void prefill_budgets_kernel(int32_t* n_valid, int32_t* k_row, int num_tiles, int total,
                                        int k_max, float pct, int rolling) {
+  pdl_begin();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   int t = i % num_tiles;
@@ -631,6 +633,7 @@ __global__ void prefill_budgets_kernel(int32_t* n_valid, int32_t* k_row, int num
 // (strategies/KascadeStrategy.py:127-139); tiles beyond a sequence's end get no candidates
 __global__ void prefill_budgets_ragged_kernel(int32_t* n_valid, int32_t* k_row, const int32_t* seq_len, int groups,
                                               int num_tiles, int total, int k_cap, float pct, int rolling) {
+  pdl_begin();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const int t = i % num_tiles, b = i / (num_tiles * groups);
@@ -657,32 +660,12 @@ extern "C" int kb200_prefill_budgets_ragged(int32_t* n_valid, int32_t* k_row, co
   KB_REQUIRE(n_valid && k_row && seq_len, "prefill_budgets_ragged: null pointer");
   int total = batch * num_kv_heads * num_tiles;
   if (total <= 0) return 0;
-  prefill_budgets_ragged_kernel<<<ceil_div(total, 256), 256, 0, (cudaStream_t)stream>>>(
-      n_valid, k_row, seq_len, num_kv_heads, num_tiles, total, k_cap, pct, rolling);
-  KB_CHECK_LAUNCH("prefill_budgets_ragged_kernel");
+  KB_CUDA(launch_pdl(prefill_budgets_ragged_kernel, dim3(ceil_div(total, 256)), 256, 0, (cudaStream_t)stream, 1, n_valid, k_row,
+                     seq_len, num_kv_heads, num_tiles, total, k_cap, pct, rolling));
   return 0;
 }
 
 namespace kb200 {
-template <int C>
-static cudaError_t topk_launch_cluster(const float* scores, int64_t row_stride, int n_cols, const int32_t* n_valid,
-                                       const int32_t* k_row, int k_max, int32_t* out_idx, int64_t idx_stride,
-                                       int32_t* out_count, int64_t rows, const DecodeBudget& budget, cudaStream_t st) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)(rows * C));
-  cfg.blockDim = dim3(kTopkThreads);
-  cfg.dynamicSmemBytes = kTopkMergedBytes;
-  cfg.stream = st;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = C;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, topk_select_kernel<C>, scores, row_stride, n_cols, n_valid, k_row, k_max, out_idx,
-                            idx_stride, out_count, rows, budget);
-}
-
 // CTAs per row: doubled while all rows together leave an SM for each CTA and a CTA keeps at least 4096 scores; below
 // that, and for rows under 16384, its fixed phases (the sample, the lists) cost more than a shorter piece saves.
 // Measured, us with one CTA / a cluster: 8 rows of 16384 / 32768 / 131072 scores 17.2 / 25.4 / 69.9 -> 15.2 / 18.5 / 27.1,
@@ -716,23 +699,11 @@ static int topk_launch(const float* scores, int64_t row_stride, int n_cols, cons
              (long long)idx_stride, k_max);
   if (rows == 0) return 0;
   cudaStream_t st = (cudaStream_t)stream;
-  switch (topk_cluster(rows, n_cols)) {
-    case 8:
-      KB_CUDA(topk_launch_cluster<8>(scores, row_stride, n_cols, n_valid, k_row, k_max, out_idx, idx_stride, out_count, rows, budget, st));
-      break;
-    case 4:
-      KB_CUDA(topk_launch_cluster<4>(scores, row_stride, n_cols, n_valid, k_row, k_max, out_idx, idx_stride, out_count, rows, budget, st));
-      break;
-    case 2:
-      KB_CUDA(topk_launch_cluster<2>(scores, row_stride, n_cols, n_valid, k_row, k_max, out_idx, idx_stride, out_count, rows, budget, st));
-      break;
-    default: {
-      const int64_t grid = rows < (int64_t)sm_count() * 64 ? rows : (int64_t)sm_count() * 64;
-      topk_select_kernel<1><<<(unsigned)grid, kTopkThreads, 0, st>>>(scores, row_stride, n_cols, n_valid, k_row, k_max, out_idx,
-                                                                     idx_stride, out_count, rows, budget);
-      KB_CHECK_LAUNCH("topk_select_kernel");
-    }
-  }
+  const int c = topk_cluster(rows, n_cols);
+  auto* kernel = c == 8 ? topk_select_kernel<8> : c == 4 ? topk_select_kernel<4> : c == 2 ? topk_select_kernel<2> : topk_select_kernel<1>;
+  const int64_t grid = c > 1 || rows < (int64_t)sm_count() * 64 ? rows * c : (int64_t)sm_count() * 64;
+  KB_CUDA(launch_pdl(kernel, dim3((unsigned)grid), kTopkThreads, c > 1 ? kTopkMergedBytes : 0, st, c, scores, row_stride, n_cols,
+                     n_valid, k_row, k_max, out_idx, idx_stride, out_count, rows, budget));
   return 0;
 }
 }  // namespace kb200
@@ -763,8 +734,7 @@ extern "C" int kb200_prefill_budgets(int32_t* n_valid, int32_t* k_row, int batch
   KB_REQUIRE(n_valid && k_row, "prefill_budgets: null pointer");
   int total = batch * num_kv_heads * num_tiles;
   if (total <= 0) return 0;
-  prefill_budgets_kernel<<<ceil_div(total, 256), 256, 0, (cudaStream_t)stream>>>(
-      n_valid, k_row, num_tiles, total, k_max, pct, rolling);
-  KB_CHECK_LAUNCH("prefill_budgets_kernel");
+  KB_CUDA(launch_pdl(prefill_budgets_kernel, dim3(ceil_div(total, 256)), 256, 0, (cudaStream_t)stream, 1, n_valid, k_row,
+                     num_tiles, total, k_max, pct, rolling));
   return 0;
 }
