@@ -31,14 +31,14 @@
 
 namespace kb200 {
 
-constexpr int kTopkThreads = 512;
-constexpr int kTopkWarps = kTopkThreads / 32;
+constexpr int kTopkWarpsMax = 16;
 constexpr int kDigit = 9;
 constexpr int kTopkBins = 1 << kDigit;                            // 9-bit digits: one warp can search a histogram
-constexpr int kCandCap = 8192;                            // keys the candidate lists hold, one list per warp
-constexpr int kWarpList = kCandCap / kTopkWarps;          // 512
+constexpr int kMergedCap = 8192;                          // keys the gathered list of a cluster holds
+// keys a warp's candidate list holds; the lists of a CTA hold 8192 together (4 warps: 4096)
+constexpr int warp_list(int warps) { return warps == 16 ? 512 : 1024; }
 constexpr int kListRow = 4096;                            // rows up to this length are selected from directly
-constexpr int kTopkMergedBytes = kCandCap * 4;            // dynamic shared memory of a cluster's CTA
+constexpr int kTopkMergedBytes = kMergedCap * 4;            // dynamic shared memory of a cluster's CTA
 constexpr int kTopkUnroll = 4;                            // 16-byte loads a lane keeps in flight in the streaming passes
 
 // order-preserving map float -> uint32 (larger float <=> larger key)
@@ -58,22 +58,24 @@ __device__ __forceinline__ void piece_keys(const float4& x, int i4, int n4, int 
   }
 }
 
+template <int NW>                      // warps of a CTA
 struct TopkShared {
   uint32_t hist[kTopkBins];
-  uint32_t cand[kCandCap];
-  uint32_t red[kTopkWarps], red2[kTopkWarps];
-  uint32_t warp_gt[kTopkWarps], warp_eq[kTopkWarps], list_len[kTopkWarps];
+  uint32_t cand[NW * warp_list(NW)];
+  uint32_t red[NW], red2[NW];
+  uint32_t warp_gt[NW], warp_eq[NW], list_len[NW];
   uint32_t digit, remaining;
   uint32_t cta_gt, cta_cand, cta_max_list;               // clusters: scores above hi_key, list entries, longest list
   uint32_t cta_above, cta_equal;                         // clusters: scores above / at the threshold in this CTA's piece
-  uint32_t list_at[8 * kTopkWarps];                      // clusters: where each list starts in the gathered one
+  uint32_t list_at[8 * kTopkWarpsMax];                   // clusters: where each list starts in the gathered one
 };
 
 // Bin d of sh.hist with  count(bins > d) < r <= count(bins >= d)  (1 <= r <= total); every thread gets d and
 // r - count(bins > d).  All threads of the CTA call it, after a barrier that completed the histogram; one warp
 // does the search (16 bins per lane) - the per-row costs of this kernel are instructions, and sixteen warps
 // searching together would issue ten times as many.
-__device__ __forceinline__ void find_bin(TopkShared& sh, uint32_t r, uint32_t& digit, uint32_t& rest) {
+template <int NW>
+__device__ __forceinline__ void find_bin(TopkShared<NW>& sh, uint32_t r, uint32_t& digit, uint32_t& rest) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (warp == 0) {
     constexpr int kPer = kTopkBins / 32;
@@ -105,27 +107,31 @@ __device__ __forceinline__ void find_bin(TopkShared& sh, uint32_t r, uint32_t& d
   __syncthreads();
 }
 
-// sum / minimum / maximum over the 16 per-warp values of an array in shared memory: one load per lane and four
-// shuffles instead of sixteen loads per thread
-__device__ __forceinline__ uint32_t warps_sum(const uint32_t* a) {
-  uint32_t v = a[threadIdx.x & (kTopkWarps - 1)];
+// sum / minimum / maximum over the per-warp values of an array in shared memory: one load per lane and a few
+// shuffles instead of a load per warp and thread
+template <int NW>
+__device__ __forceinline__ uint32_t warps_sum(const uint32_t (&a)[NW]) {
+  uint32_t v = a[threadIdx.x & (NW - 1)];
 #pragma unroll
-  for (int off = kTopkWarps / 2; off > 0; off >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, off);
+  for (int off = NW / 2; off > 0; off >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, off);
   return v;
 }
-__device__ __forceinline__ uint32_t warps_min(const uint32_t* a) {
-  uint32_t v = a[threadIdx.x & (kTopkWarps - 1)];
+template <int NW>
+__device__ __forceinline__ uint32_t warps_min(const uint32_t (&a)[NW]) {
+  uint32_t v = a[threadIdx.x & (NW - 1)];
 #pragma unroll
-  for (int off = kTopkWarps / 2; off > 0; off >>= 1) v = min(v, __shfl_xor_sync(0xFFFFFFFFu, v, off));
+  for (int off = NW / 2; off > 0; off >>= 1) v = min(v, __shfl_xor_sync(0xFFFFFFFFu, v, off));
   return v;
 }
-__device__ __forceinline__ uint32_t warps_max(const uint32_t* a) {
-  uint32_t v = a[threadIdx.x & (kTopkWarps - 1)];
+template <int NW>
+__device__ __forceinline__ uint32_t warps_max(const uint32_t (&a)[NW]) {
+  uint32_t v = a[threadIdx.x & (NW - 1)];
 #pragma unroll
-  for (int off = kTopkWarps / 2; off > 0; off >>= 1) v = max(v, __shfl_xor_sync(0xFFFFFFFFu, v, off));
+  for (int off = NW / 2; off > 0; off >>= 1) v = max(v, __shfl_xor_sync(0xFFFFFFFFu, v, off));
   return v;
 }
-__device__ __forceinline__ uint32_t block_sum(TopkShared& sh, uint32_t v) {
+template <int NW>
+__device__ __forceinline__ uint32_t block_sum(TopkShared<NW>& sh, uint32_t v) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, off);
@@ -150,16 +156,15 @@ __device__ __forceinline__ int decode_budget(const DecodeBudget& d, int n) {
   return min(max(128, (int)(d.share * (double)n)), n) - d.tile;
 }
 
-#ifndef KB200_TOPK_MIN_CTAS
-#define KB200_TOPK_MIN_CTAS 2      // CTAs per SM the register allocation aims at (3, with a few spills, measured no faster)
-#endif
-template <int C>                       // CTAs that share a row (a cluster of C)
-__global__ void __launch_bounds__(kTopkThreads, KB200_TOPK_MIN_CTAS)
+template <int C, int kTopkWarps>       // CTAs that share a row (a cluster of C), warps per CTA
+__global__ void __launch_bounds__(kTopkWarps * 32, 32 / kTopkWarps)
 topk_select_kernel(const float* __restrict__ scores, int64_t row_stride, int n_cols,
                    const int32_t* __restrict__ n_valid, const int32_t* __restrict__ k_row, int k_max,
                    int32_t* __restrict__ out_idx, int64_t idx_stride, int32_t* __restrict__ out_count,
                    int64_t rows, const DecodeBudget budget) {
   namespace cg = cooperative_groups;
+  using TopkShared = TopkShared<kTopkWarps>;
+  constexpr int kTopkThreads = kTopkWarps * 32, kWarpList = warp_list(kTopkWarps);
   __shared__ TopkShared sh;
   extern __shared__ uint32_t merged[];                    // C > 1: the lists of all CTAs of the cluster
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -198,13 +203,15 @@ topk_select_kernel(const float* __restrict__ scores, int64_t row_stride, int n_c
     uint32_t lo_key = 0u, hi_key = 0xFFFFFFFFu;
     const bool sampled = n > kListRow;
     if (sampled) {
-      const int f4 = n > 65536 ? 4 : 2;                  // 16-byte pieces per thread: 4096 or 8192 sampled scores
+      constexpr int kF4 = 1024 / kTopkThreads;           // 16-byte pieces per thread that make 4096 sampled scores
+      constexpr int kMaxF4 = kTopkWarps == 4 ? kF4 : 2 * kF4;
+      const int f4 = n > 65536 ? kMaxF4 : kF4;           // 8192 for long rows (four warps are not given those)
       const int n_samp = f4 * kTopkThreads * 4;
-      uint32_t sk[16], smin = 0xFFFFFFFFu, smax = 0u;
+      uint32_t sk[4 * kMaxF4], smin = 0xFFFFFFFFu, smax = 0u;
 #pragma unroll
-      for (int it = 0; it < 4; ++it) {
+      for (int it = 0; it < kMaxF4; ++it) {
         if (it < f4) {
-          const int pos = (int)(((int64_t)(it * kTopkThreads + tid) * n4) >> (f4 == 4 ? 11 : 10));  // < n4 - 1
+          const int pos = (int)(((int64_t)(it * kTopkThreads + tid) * n4) >> (f4 == kF4 ? 10 : 11));  // < n4 - 1
           const float4 x = __ldg(row4 + pos);
           sk[it * 4 + 0] = float_key(x.x); sk[it * 4 + 1] = float_key(x.y);
           sk[it * 4 + 2] = float_key(x.z); sk[it * 4 + 3] = float_key(x.w);
@@ -213,7 +220,7 @@ topk_select_kernel(const float* __restrict__ scores, int64_t row_stride, int n_c
         }
       }
 #pragma unroll
-      for (int i = 0; i < 16; ++i) { smin = min(smin, sk[i]); smax = max(smax, sk[i]); }
+      for (int i = 0; i < 4 * kMaxF4; ++i) { smin = min(smin, sk[i]); smax = max(smax, sk[i]); }
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) {
         smin = min(smin, __shfl_xor_sync(0xFFFFFFFFu, smin, off));
@@ -232,10 +239,10 @@ topk_select_kernel(const float* __restrict__ scores, int64_t row_stride, int n_c
         const uint32_t range = top - bottom;
         const int shift = (range >> kDigit) ? (32 - __clz(range) - kDigit) : 0;      // (range >> shift) < kTopkBins
 #pragma unroll
-        for (int i = 0; i < 8; ++i) atomicAdd(&sh.hist[(sk[i] - bottom) >> shift], 1u);
-        if (f4 == 4) {
+        for (int i = 0; i < 4 * kF4; ++i) atomicAdd(&sh.hist[(sk[i] - bottom) >> shift], 1u);
+        if (f4 != kF4) {
 #pragma unroll
-          for (int i = 8; i < 16; ++i) atomicAdd(&sh.hist[(sk[i] - bottom) >> shift], 1u);
+          for (int i = 4 * kF4; i < 4 * kMaxF4; ++i) atomicAdd(&sh.hist[(sk[i] - bottom) >> shift], 1u);
         }
         __syncthreads();
         uint32_t b, rest;
@@ -258,15 +265,15 @@ topk_select_kernel(const float* __restrict__ scores, int64_t row_stride, int n_c
         __syncthreads();
         uint32_t inside = 0;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < 4 * kF4; ++i) {
           if (sk[i] - z_lo <= range) {                     // z_lo <= key <= z_hi
             atomicAdd(&sh.hist[(sk[i] - z_lo) >> shift], 1u);
             ++inside;
           }
         }
-        if (f4 == 4) {
+        if (f4 != kF4) {
 #pragma unroll
-          for (int i = 8; i < 16; ++i) {
+          for (int i = 4 * kF4; i < 4 * kMaxF4; ++i) {
             if (sk[i] - z_lo <= range) {
               atomicAdd(&sh.hist[(sk[i] - z_lo) >> shift], 1u);
               ++inside;
@@ -365,7 +372,7 @@ topk_select_kernel(const float* __restrict__ scores, int64_t row_stride, int n_c
         n_cand += peer->cta_cand;
         fits = fits && peer->cta_max_list <= (uint32_t)kWarpList;
       }
-      fits = fits && n_cand <= (uint32_t)kCandCap;
+      fits = fits && n_cand <= (uint32_t)kMergedCap;
       if (fits) {                                         // (the same for the whole cluster)
         if (warp == 0) {                                  // C / 2 lists per lane
           constexpr int kPer = C * kTopkWarps / 32;
@@ -678,10 +685,21 @@ static int topk_cluster(int64_t rows, int n_cols) {
   return c;
 }
 
+// Warps of a CTA that has a row to itself.  A row's serial phases (some thirty CTA barriers) are what bounds this kernel
+// when there are many rows, so smaller CTAs, of which more are resident at two thousand threads per SM, hide more of
+// them.  Few rows want many warps each, and rows that do not fit the lists of four warps (about 65536 scores) at least
+// eight.  Measured, us with 16 / 8 / 4 warps: 512 prompt rows of up to 2048 scores 18.2 / 12.6 / 12.5, 3008 x 3001 88 / 50 / 40,
+// 2048 x 8192 92 / 63 / 58, 8192 x 32768 626 / 490 / 505, 24576 x 98304 3776 / 3428 / 7405; decode rows 512 x 32768
+// 68 / 61 / 77, 256 x 16000 23 / 25 / 37, 192 x 65536 58 / 73 / 435.
+static int topk_warps(int64_t rows, int n_cols) {
+  if (rows < 3ll * sm_count()) return 16;
+  return n_cols <= 8192 ? 4 : 8;
+}
+
 int init_topk() {
-  KB_CUDA(cudaFuncSetAttribute(topk_select_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTopkMergedBytes));
-  KB_CUDA(cudaFuncSetAttribute(topk_select_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTopkMergedBytes));
-  KB_CUDA(cudaFuncSetAttribute(topk_select_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTopkMergedBytes));
+  KB_CUDA(cudaFuncSetAttribute(topk_select_kernel<2, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTopkMergedBytes));
+  KB_CUDA(cudaFuncSetAttribute(topk_select_kernel<4, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTopkMergedBytes));
+  KB_CUDA(cudaFuncSetAttribute(topk_select_kernel<8, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTopkMergedBytes));
   return 0;
 }
 
@@ -700,10 +718,17 @@ static int topk_launch(const float* scores, int64_t row_stride, int n_cols, cons
   if (rows == 0) return 0;
   cudaStream_t st = (cudaStream_t)stream;
   const int c = topk_cluster(rows, n_cols);
-  auto* kernel = c == 8 ? topk_select_kernel<8> : c == 4 ? topk_select_kernel<4> : c == 2 ? topk_select_kernel<2> : topk_select_kernel<1>;
-  const int64_t grid = c > 1 || rows < (int64_t)sm_count() * 64 ? rows * c : (int64_t)sm_count() * 64;
-  KB_CUDA(launch_pdl(kernel, dim3((unsigned)grid), kTopkThreads, c > 1 ? kTopkMergedBytes : 0, st, c, scores, row_stride, n_cols,
-                     n_valid, k_row, k_max, out_idx, idx_stride, out_count, rows, budget));
+  auto* kernel = topk_select_kernel<1, 16>;
+  int warps = 16;
+  if (c == 1) {
+    warps = topk_warps(rows, n_cols);
+    kernel = warps == 4 ? topk_select_kernel<1, 4> : warps == 8 ? topk_select_kernel<1, 8> : topk_select_kernel<1, 16>;
+  } else {
+    kernel = c == 8 ? topk_select_kernel<8, 16> : c == 4 ? topk_select_kernel<4, 16> : topk_select_kernel<2, 16>;
+  }
+  const int64_t most = (int64_t)sm_count() * 1024 / warps;
+  KB_CUDA(launch_pdl(kernel, dim3((unsigned)(c > 1 || rows < most ? rows * c : most)), warps * 32, c > 1 ? kTopkMergedBytes : 0, st,
+                     c, scores, row_stride, n_cols, n_valid, k_row, k_max, out_idx, idx_stride, out_count, rows, budget));
   return 0;
 }
 }  // namespace kb200

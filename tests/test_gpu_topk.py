@@ -172,10 +172,12 @@ def test_decode_selection_rejects_bad_arguments():
 
 
 @pytest.mark.parametrize("rows,n", [(1, 8191), (1, 8192), (1, 16384), (3, 32768), (8, 131071), (37, 33000), (38, 33000), (74, 16400),
-                                    (75, 16400), (148, 9000), (149, 9000)])
+                                    (75, 16400), (148, 16400), (149, 16400), (444, 700), (444, 3001), (444, 8192), (444, 8193),
+                                    (444, 40001)])
 @pytest.mark.parametrize("kind", ["smooth", "ties", "steps"])
-def test_rows_shared_by_a_cluster(rows, n, kind):
-    """Few long rows are split over the CTAs of a cluster (2, 4 or 8, by rows and columns).  The selection is exact, so it
+def test_any_number_of_threads_selects_the_same(rows, n, kind):
+    """Few long rows are split over the CTAs of a cluster (2, 4 or 8, by rows and columns), many rows get CTAs of 4 or 8
+    warps each.  The selection is exact, so it
     equals a stable sort's, ties from the lowest index, whatever the number of CTAs: also where the sample's bracket
     fails (`ties`: half of the row has one value; `steps`: four values) and where single rows are short, empty or
     selected as a whole."""
