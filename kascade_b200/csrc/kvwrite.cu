@@ -81,6 +81,21 @@ __global__ void __launch_bounds__(kKvWriteThreads) kv_write_kernel(const KvWrite
   const int b = blockIdx.x / p.T, t = blockIdx.x - b * p.T;
   const int n = p.n_new ? p.n_new[b] : p.T;
   if (t >= n) return;
+  const int heads = p.H + 2 * p.G;                                   // Q heads, K heads, V heads
+  const int c = lane & 7;
+  // The rows a warp takes next are loaded before the current ones are worked on, the first ones before sin and cos: a
+  // CTA lives for two or three such steps only, so a load that waits for the step before it is time without traffic.
+  auto load_rows = [&](int h0, uint4& lo, uint4& hi) {
+    const int h = min(h0 + (lane >> 3), heads - 1);
+    const __half* src = h < p.H ? p.q_in + b * p.q_sb + t * p.q_st + h * p.q_sh
+                      : h < p.H + p.G ? p.k_new + b * p.k_sb + t * p.k_st + (h - p.H) * p.k_sh
+                                      : p.v_new + b * p.v_sb + t * p.v_st + (h - p.H - p.G) * p.v_sh;
+    lo = reinterpret_cast<const uint4*>(src)[c];                     // elements 8c .. 8c+7
+    hi = reinterpret_cast<const uint4*>(src + kD / 2)[c];            // elements 64+8c .. 64+8c+7
+  };
+  constexpr int kStep = (kKvWriteThreads / 32) * 4;
+  uint4 next_lo = make_uint4(0u, 0u, 0u, 0u), next_hi = next_lo;
+  if (warp * 4 < heads) load_rows(warp * 4, next_lo, next_hi);
   const int pos = p.start_pos[b] + t;
   if (p.inv_freq && tid < kD / 2) {
     float sn, cs;
@@ -89,18 +104,13 @@ __global__ void __launch_bounds__(kKvWriteThreads) kv_write_kernel(const KvWrite
     sin_s[tid] = from_f<BF16>(sn * p.rope_scale);
   }
   __syncthreads();
-  const int heads = p.H + 2 * p.G;                                   // Q heads, K heads, V heads
-  const int c = lane & 7;
-  for (int h0 = warp * 4; h0 < heads; h0 += (kKvWriteThreads / 32) * 4) {   // uniform per warp
+  for (int h0 = warp * 4; h0 < heads; h0 += kStep) {                 // uniform per warp
     const int h = min(h0 + (lane >> 3), heads - 1);
     const bool active = h0 + (lane >> 3) < heads;                    // the last group of rows may be partial
     const int kind = h < p.H ? 0 : (h < p.H + p.G ? 1 : 2);          // 0 = Q, 1 = K, 2 = V
     const int hh = kind == 0 ? h : (kind == 1 ? h - p.H : h - p.H - p.G);
-    const __half* src = kind == 0 ? p.q_in + b * p.q_sb + t * p.q_st + hh * p.q_sh
-                      : kind == 1 ? p.k_new + b * p.k_sb + t * p.k_st + hh * p.k_sh
-                                  : p.v_new + b * p.v_sb + t * p.v_st + hh * p.v_sh;
-    uint4 lo4 = reinterpret_cast<const uint4*>(src)[c];              // elements 8c .. 8c+7
-    uint4 hi4 = reinterpret_cast<const uint4*>(src + kD / 2)[c];     // elements 64+8c .. 64+8c+7
+    uint4 lo4 = next_lo, hi4 = next_hi;
+    if (h0 + kStep < heads) load_rows(h0 + kStep, next_lo, next_hi);
     H2* lo = reinterpret_cast<H2*>(&lo4);
     H2* hi = reinterpret_cast<H2*>(&hi4);
     const __half* gain = kind == 0 ? p.q_gain : (kind == 1 ? p.k_gain : nullptr);
