@@ -286,6 +286,10 @@ int kb200_prefill_sparse_ragged(const kb200_act_layout* q, const kb200_act_layou
 int kb200_prefill_budgets_ragged(int32_t* n_valid, int32_t* k_row, const int32_t* seq_len, int batch,
                                  int num_kv_heads, int num_tiles, int k_cap, float pct, int rolling, void* stream);
 
+/* Zeros the rows of out [batch, max_len, row_bytes] that lie outside the sequences of a ragged batch (the ragged
+ * prefill calls write only the rows inside). */
+int kb200_zero_padding(void* out, const kb200_ragged* ragged, int batch, int max_len, int64_t row_bytes, void* stream);
+
 /* Output fan-out for prompts whose KV heads are sharded over GPUs: the rows a call computes (its
  * num_q_heads heads) are stored by the kernel's epilogue into `count` buffers, each
  * [B, L, total_heads, D] fp16 contiguous, at heads [head_offset, head_offset + num_q_heads).  out[0] is

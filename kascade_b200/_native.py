@@ -29,7 +29,7 @@ EXPORTS = [
     "kb200_prefill_sparse", "kb200_prefill_budgets", "kb200_selftest_umma", "kb200_read_status",
     "kb200_decode_sparse_paged_noalloc", "kb200_prefill_dense_fanout", "kb200_prefill_sparse_fanout",
     "kb200_kv_write", "kb200_prefill_dense_ragged", "kb200_prefill_pool_scores_ragged", "kb200_prefill_sparse_ragged",
-    "kb200_prefill_budgets_ragged", "kb200_peer_push", "kb200_stream_wait_events", "kb200_selftest_wait_timeout", "kb200_tensor_map_encodes", "kb200_decode_noalloc_splits",
+    "kb200_prefill_budgets_ragged", "kb200_zero_padding", "kb200_peer_push", "kb200_stream_wait_events", "kb200_selftest_wait_timeout", "kb200_tensor_map_encodes", "kb200_decode_noalloc_splits",
 ]
 
 
@@ -143,6 +143,7 @@ def load() -> C.CDLL:
         lib.kb200_prefill_sparse_ragged.argtypes = [AL, AL, AL, vp, i64, vp, vp, f32, vp, vp, RG, i32, i32, i32,
                                                     i32, i32, vp]
         lib.kb200_prefill_budgets_ragged.argtypes = [vp, vp, vp, i32, i32, i32, i32, f32, i32, vp]
+        lib.kb200_zero_padding.argtypes = [vp, RG, i32, i32, i64, vp]
         lib.kb200_kv_write.argtypes = [AL, vp, AL, AL, vp, vp, C.POINTER(KvLayout), vp, vp, f32, vp, f32, i32, i32,
                                        i32, i32, vp]
         lib.kb200_selftest_umma.argtypes = [vp, vp, vp, vp, vp]
@@ -489,6 +490,18 @@ def prefill_dense(q, k, v, scale, out, lse2, fanout: Optional[OutFanout] = None,
     _check(lib.kb200_prefill_dense(C.byref(ql), C.byref(kl), C.byref(vl), float(scale), _ptr(out), _ptr(lse2),
                                    B, L, H, G, _stream()), "kb200_prefill_dense")
     _launched(1)
+
+
+@_on_device_of(0)
+def zero_padding(out: torch.Tensor, ragged: Ragged):
+    """Zeros the rows of out [B, L, ...] (contiguous) that lie outside the sequences."""
+    lib = init(out.get_device())
+    assert out.is_contiguous()
+    B, L = out.shape[:2]
+    if out.numel() == 0:
+        return
+    _check(lib.kb200_zero_padding(_ptr(out), C.byref(ragged), B, L, out.numel() * out.element_size() // (B * L), _stream()),
+           "kb200_zero_padding")                     # (stands for a memset: not in launch_count)
 
 
 @_on_device_of(0)

@@ -1274,6 +1274,23 @@ selftest_wait_timeout_kernel(int32_t* __restrict__ result, unsigned long long li
   }
 }
 
+// Rows outside the sequences of a ragged batch: zeros.  One CTA per kPadRows consecutive rows of a slot; rows inside a
+// sequence are left alone, so only the padding is written (bound by HBM writes; clearing the whole output first took
+// 26 us per layer at 4 x 3001 tokens, as much as a quarter of the sparse kernel after it).
+constexpr int kPadRows = 8;
+__global__ void __launch_bounds__(256) zero_padding_kernel(uint4* __restrict__ out, const int32_t* __restrict__ seq_start,
+                                                           const int32_t* __restrict__ seq_len, int max_len, int row16) {
+  const int b = blockIdx.y;
+  const int begin = seq_start ? seq_start[b] : 0, end = begin + max(seq_len[b], 0);
+  const int r0 = blockIdx.x * kPadRows, r1 = min(r0 + kPadRows, max_len);
+  if (r0 >= begin && r1 <= end) return;
+  for (int r = r0; r < r1; ++r) {
+    if (r >= begin && r < end) continue;
+    uint4* row = out + ((int64_t)b * max_len + r) * row16;
+    for (int i = threadIdx.x; i < row16; i += 256) row[i] = make_uint4(0u, 0u, 0u, 0u);
+  }
+}
+
 // ---- host side ---------------------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -1665,4 +1682,20 @@ extern "C" int kb200_prefill_sparse_ragged(const kb200_act_layout* q, const kb20
   KB_REQUIRE(ragged, "prefill_sparse_ragged: ragged is null");
   return prefill_sparse_impl(q, k, v, tile_idx, idx_stride, tile_count, head_map, softmax_scale, out, nullptr, lse2,
                              batch, max_len, num_q_heads, num_kv_heads, idx_kv_heads, stream, ragged);
+}
+
+extern "C" int kb200_zero_padding(void* out, const kb200_ragged* ragged, int batch, int max_len, int64_t row_bytes,
+                                  void* stream) {
+  using namespace kb200;
+  KB_ENTRY(out, "zero_padding: out");
+  KB_REQUIRE(out && ragged && ragged->seq_len, "zero_padding: null pointer");
+  KB_REQUIRE(batch >= 0 && batch <= 65535 && max_len >= 0, "zero_padding: batch %d, %d rows", batch, max_len);
+  KB_REQUIRE(row_bytes > 0 && row_bytes % 16 == 0 && row_bytes / 16 < (1ll << 30) &&
+                 (reinterpret_cast<uintptr_t>(out) & 15) == 0,
+             "zero_padding: rows must be 16-byte aligned");
+  if (batch == 0 || max_len == 0) return 0;
+  zero_padding_kernel<<<dim3(ceil_div(max_len, kPadRows), batch), 256, 0, (cudaStream_t)stream>>>(
+      static_cast<uint4*>(out), ragged->seq_start, ragged->seq_len, max_len, (int)(row_bytes / 16));
+  KB_CHECK_LAUNCH("zero_padding_kernel");
+  return 0;
 }

@@ -367,10 +367,10 @@ class EfficientKascadeStrategy(Strategy):
                 out.zero_()
         elif fan is not None:
             out = None
-        elif rg is not None:
-            out = torch.zeros(B, L, H, D, dtype=q.dtype, device=dev)
         else:
             out = torch.empty(B, L, H, D, dtype=q.dtype, device=dev)
+            if rg is not None:
+                nat.zero_padding(out, rg)
         if self.is_anchor(layer):
             kk = topk_budget(self.k, L, self.tile_size) if ragged is None else \
                 max(1, max(topk_budget(self.k, n, self.tile_size) for n in ragged[2]))

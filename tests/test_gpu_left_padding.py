@@ -118,3 +118,23 @@ def test_unpadded_mask_takes_the_batched_path():
     assert s._padding(None, 2, 64) is None
     assert s._padding(_mask([0, 5], 64, 64), 2, 64) == ([0, 5], [64, 59])
     assert s._padding(_mask([0, 5], 64, 64, right=[10, 0]), 2, 64) == ([0, 5], [54, 59])
+
+
+@pytest.mark.parametrize("L", [1, 8, 9, 64, 129])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_zero_padding_clears_exactly_the_rows_outside(L, dtype):
+    """Sequences that fill their slot, are empty, start or end inside a group of rows, or are given without first rows."""
+    from kascade_b200 import _native as nat
+    dev = torch.device("cuda")
+    starts = [0, 0, min(3, L - 1), L - 1, L // 2]
+    lens = [L, 0, max(L - 3 - (L > 8), 0), 1, L - L // 2]
+    for first in (starts, None):
+        out = torch.full((len(lens), L, 5, 8), 7.0, dtype=dtype, device=dev)
+        rg = (None if first is None else torch.tensor(first, dtype=torch.int32, device=dev),
+              torch.tensor(lens, dtype=torch.int32, device=dev))
+        nat.zero_padding(out, nat.ragged(*rg))
+        pos = torch.arange(L)
+        for b, n in enumerate(lens):
+            s = 0 if first is None else first[b]
+            inside = (pos >= s) & (pos < s + n)
+            assert bool((out[b].cpu()[inside] == 7).all()) and bool((out[b].cpu()[~inside] == 0).all()), (L, b)
