@@ -246,3 +246,41 @@ def test_mixed_batch_short_sequences_attend_to_everything():
         p = torch.softmax(torch.einsum("ghd,gld->ghl", qb, kb) * scale, -1)
         ref = torch.einsum("ghl,gld->ghd", p, vb).reshape(H, D)
         assert_close(whole[1][b], ref, what=f"short sequence {b} against dense attention")
+
+
+@pytest.mark.parametrize("has_v", [True, False])
+def test_dense_decode_takes_the_longest_sequences_first(has_v):
+    """A dense pass of more CTAs than the chip holds, of 8192 keys or more each, hands out up to 32 sequences by length.
+    Order is all that changes: with one sequence more, which are taken as they come, every sequence gives the same bits -
+    among them equal lengths, the longest one last, one key and none."""
+    from kascade_b200 import _native as nat
+    g = torch.Generator(device="cuda").manual_seed(5)
+    lens = [300, 16384, 0, 1, 9000, 300, 5000, 16384] + [100 + 37 * i for i in range(23)] + [16390]
+    B, G, H, D, page, splits = len(lens), 8, 32, 128, 16, 2
+    assert B == 32 and B * G * splits > 2 * nat.sm_count(0) and max(lens) // splits >= 8192
+    pages = [-(-n // page) for n in lens]
+    shape = (sum(pages) + 1, page, G, D)
+    k = torch.randn(shape, generator=g, device="cuda").half()
+    v = torch.randn(shape, generator=g, device="cuda").half()
+    q = torch.randn(B, H, D, generator=g, device="cuda").half()
+    table = torch.zeros(B, max(pages), dtype=torch.int32)
+    at = 0
+    for b, n in enumerate(pages):
+        table[b, :n] = torch.arange(at, at + n)
+        at += n
+    table, seq_lens = table.cuda(), torch.tensor(lens, dtype=torch.int32, device="cuda")
+    stride = -(-max(lens) // 4) * 4
+
+    def run(rows):
+        n = len(rows)
+        out = torch.zeros(n, H, D, dtype=torch.float16, device="cuda") if has_v else None
+        logits, pooled = torch.zeros(n, H, stride, device="cuda"), torch.zeros(n, G, stride, device="cuda")
+        lse2 = torch.zeros(n, H, device="cuda")
+        kv = nat.kv_layout_paged(k, v if has_v else None, table[rows].contiguous())
+        nat.decode_anchor_paged(q[rows].contiguous(), kv, seq_lens[rows].contiguous(), max(lens), D ** -0.5, logits, pooled,
+                                out, lse2, nat.decode_workspace(n, H, splits, "cuda"), splits)
+        return [x for x in (out, lse2, logits, pooled) if x is not None]
+
+    for got, want in zip(run(list(range(B))), run(list(range(B)) + [0])):      # 33 sequences are not ranked
+        for b in range(B):
+            assert torch.equal(got[b], want[b]), f"sequence {b} of {lens[b]} keys"
