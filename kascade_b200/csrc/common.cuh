@@ -38,6 +38,19 @@ int check_on_current_device(const void* ptr, const char* what);
     }                                                                            \
   } while (0)
 
+// The check of a kernel launch: KB_LAUNCH of one that returns its error, KB_CHECK_LAUNCH after one with <<<>>>.  A launch that
+// the runtime refuses is also left behind as its last error; both take it back, so that the next launch check in this
+// thread (PyTorch's, for one) does not report it a second time.
+#define KB_LAUNCH(name, launch)                                                  \
+  do {                                                                           \
+    const cudaError_t launched__ = (launch);                                     \
+    if (launched__ != cudaSuccess) {                                             \
+      cudaGetLastError();                                                        \
+      kb200::set_error("launch of %s failed: %s", name, cudaGetErrorString(launched__)); \
+      return -1;                                                                 \
+    }                                                                            \
+  } while (0)
+
 #define KB_CHECK_LAUNCH(name)                                                    \
   do {                                                                           \
     cudaError_t e__ = cudaGetLastError();                                        \

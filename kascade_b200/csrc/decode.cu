@@ -776,8 +776,8 @@ extern "C" int kb200_decode_sparse_paged(const void* q, int64_t q_stride_b, int6
   if (p.fp8) rc = launch_attn<false, true, false, 2>(p, grid, k_max, st);
   else if (p.bf16) rc = launch_attn<false, true, false, 1>(p, grid, k_max, st);
   else rc = launch_attn<false, true, false, 0>(p, grid, k_max, st);
-  KB_CUDA(rc);
-  if (splits > 1) KB_CUDA(launch_combine(p, true, batch, st));
+  KB_LAUNCH("decode_attn_kernel<sparse>", rc);
+  if (splits > 1) KB_LAUNCH("decode_combine_kernel", launch_combine(p, true, batch, st));
   return 0;
 }
 
@@ -831,12 +831,12 @@ extern "C" int kb200_decode_anchor_paged(const void* q, int64_t q_stride_b, int6
   else if (p.fp8) rc = launch_attn<true, false, true, 2>(p, grid, max_seq_len, st);
   else if (p.bf16) rc = launch_attn<true, false, true, 1>(p, grid, max_seq_len, st);
   else rc = launch_attn<true, false, true, 0>(p, grid, max_seq_len, st);
-  KB_CUDA(rc);
-  if (splits > 1) KB_CUDA(launch_combine(p, has_v, batch, st));
+  KB_LAUNCH("decode_attn_kernel<dense>", rc);
+  if (splits > 1) KB_LAUNCH("decode_combine_kernel", launch_combine(p, has_v, batch, st));
   if (max_seq_len > 0) {
     dim3 pgrid(ceil_div(max_seq_len, 1024), num_kv_heads, batch);
-    KB_CUDA(launch_pdl(decode_pool_kernel, pgrid, 256, 0, st, 1, logits, lse2_out, seq_lens, pooled, logit_stride,
-                       num_q_heads, num_kv_heads));
+    KB_LAUNCH("decode_pool_kernel", launch_pdl(decode_pool_kernel, pgrid, 256, 0, st, 1, logits, lse2_out, seq_lens, pooled,
+                                               logit_stride, num_q_heads, num_kv_heads));
   }
   return 0;
 }
@@ -898,7 +898,7 @@ extern "C" int kb200_decode_sparse_paged_noalloc(const void* q, int64_t q_stride
   if (p.fp8) rc = launch_attn<false, true, false, 2>(p, grid, k_max, st);
   else if (p.bf16) rc = launch_attn<false, true, false, 1>(p, grid, k_max, st);
   else rc = launch_attn<false, true, false, 0>(p, grid, k_max, st);
-  KB_CUDA(rc);
-  if (splits > 1) KB_CUDA(launch_combine(p, true, batch, st));
+  KB_LAUNCH("decode_attn_kernel<sparse, noalloc>", rc);
+  if (splits > 1) KB_LAUNCH("decode_combine_kernel<noalloc>", launch_combine(p, true, batch, st));
   return 0;
 }

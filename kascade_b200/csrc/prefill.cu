@@ -1524,7 +1524,7 @@ static int prefill_dense_impl(const kb200_act_layout* q, const kb200_act_layout*
     rc = launch_pdl(tile_prefill_kernel<kDenseLse, true>, grid, PfCfg<kDenseLse>::kThreads, kSmemNoV, (cudaStream_t)stream, 1, p, tq, tk, tv);
   else
     rc = launch_pdl(tile_prefill_kernel<kDenseLse, false>, grid, PfCfg<kDenseLse>::kThreads, kSmemNoV, (cudaStream_t)stream, 1, p, tq, tk, tv);
-  KB_CUDA(rc);
+  KB_LAUNCH("tile_prefill_kernel<dense>", rc);
   return 0;
 }
 }  // namespace kb200
@@ -1575,7 +1575,7 @@ static int prefill_pool_impl(const kb200_act_layout* q, const kb200_act_layout* 
     rc = launch_pdl(tile_prefill_kernel<kPool, true>, grid, PfCfg<kPool>::kThreads, kSmemNoV, (cudaStream_t)stream, 1, p, tq, tk, tk);
   else
     rc = launch_pdl(tile_prefill_kernel<kPool, false>, grid, PfCfg<kPool>::kThreads, kSmemNoV, (cudaStream_t)stream, 1, p, tq, tk, tk);
-  KB_CUDA(rc);
+  KB_LAUNCH("tile_prefill_kernel<pool>", rc);
   return 0;
 }
 }  // namespace kb200
@@ -1648,7 +1648,7 @@ static int prefill_sparse_impl(const kb200_act_layout* q, const kb200_act_layout
     rc = launch_pdl(tile_prefill_kernel<kSparse, true>, grid, PfCfg<kSparse>::kThreads, kSmemAttn, (cudaStream_t)stream, 1, p, tq, none, none);
   else
     rc = launch_pdl(tile_prefill_kernel<kSparse, false>, grid, PfCfg<kSparse>::kThreads, kSmemAttn, (cudaStream_t)stream, 1, p, tq, none, none);
-  KB_CUDA(rc);
+  KB_LAUNCH("tile_prefill_kernel<sparse>", rc);
   return 0;
 }
 }  // namespace kb200

@@ -667,8 +667,9 @@ extern "C" int kb200_prefill_budgets_ragged(int32_t* n_valid, int32_t* k_row, co
   KB_REQUIRE(n_valid && k_row && seq_len, "prefill_budgets_ragged: null pointer");
   int total = batch * num_kv_heads * num_tiles;
   if (total <= 0) return 0;
-  KB_CUDA(launch_pdl(prefill_budgets_ragged_kernel, dim3(ceil_div(total, 256)), 256, 0, (cudaStream_t)stream, 1, n_valid, k_row,
-                     seq_len, num_kv_heads, num_tiles, total, k_cap, pct, rolling));
+  KB_LAUNCH("prefill_budgets_ragged_kernel",
+            launch_pdl(prefill_budgets_ragged_kernel, dim3(ceil_div(total, 256)), 256, 0, (cudaStream_t)stream, 1, n_valid,
+                       k_row, seq_len, num_kv_heads, num_tiles, total, k_cap, pct, rolling));
   return 0;
 }
 
@@ -727,8 +728,10 @@ static int topk_launch(const float* scores, int64_t row_stride, int n_cols, cons
     kernel = c == 8 ? topk_select_kernel<8, 16> : c == 4 ? topk_select_kernel<4, 16> : topk_select_kernel<2, 16>;
   }
   const int64_t most = (int64_t)sm_count() * 1024 / warps;
-  KB_CUDA(launch_pdl(kernel, dim3((unsigned)(c > 1 || rows < most ? rows * c : most)), warps * 32, c > 1 ? kTopkMergedBytes : 0, st,
-                     c, scores, row_stride, n_cols, n_valid, k_row, k_max, out_idx, idx_stride, out_count, rows, budget));
+  const dim3 grid((unsigned)(c > 1 || rows < most ? rows * c : most));
+  KB_LAUNCH("topk_select_kernel",
+            launch_pdl(kernel, grid, warps * 32, c > 1 ? kTopkMergedBytes : 0, st, c, scores, row_stride, n_cols, n_valid, k_row,
+                       k_max, out_idx, idx_stride, out_count, rows, budget));
   return 0;
 }
 }  // namespace kb200
@@ -759,7 +762,8 @@ extern "C" int kb200_prefill_budgets(int32_t* n_valid, int32_t* k_row, int batch
   KB_REQUIRE(n_valid && k_row, "prefill_budgets: null pointer");
   int total = batch * num_kv_heads * num_tiles;
   if (total <= 0) return 0;
-  KB_CUDA(launch_pdl(prefill_budgets_kernel, dim3(ceil_div(total, 256)), 256, 0, (cudaStream_t)stream, 1, n_valid, k_row,
-                     num_tiles, total, k_max, pct, rolling));
+  KB_LAUNCH("prefill_budgets_kernel",
+            launch_pdl(prefill_budgets_kernel, dim3(ceil_div(total, 256)), 256, 0, (cudaStream_t)stream, 1, n_valid, k_row,
+                       num_tiles, total, k_max, pct, rolling));
   return 0;
 }

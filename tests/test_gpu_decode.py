@@ -284,3 +284,32 @@ def test_dense_decode_takes_the_longest_sequences_first(has_v):
     for got, want in zip(run(list(range(B))), run(list(range(B)) + [0])):      # 33 sequences are not ranked
         for b in range(B):
             assert torch.equal(got[b], want[b]), f"sequence {b} of {lens[b]} keys"
+
+
+@pytest.mark.parametrize("entry", ["sparse", "noalloc", "anchor"])
+def test_a_refused_launch_names_its_kernel_and_leaves_no_error_behind(entry):
+    """65536 sequences exceed a grid's third dimension: the runtime refuses the launch before anything runs.  The call says
+    which kernel it was, and the next launches - PyTorch's and this library's - do not find the error of this one."""
+    from kascade_b200 import _native as nat
+    dev = torch.device("cuda")
+    G, H, D = 1, 4, 128
+    cache = torch.zeros(1, 16, G, D, dtype=torch.float16, device=dev)
+
+    def call(B):
+        q, out = (torch.zeros(B, H, D, dtype=torch.float16, device=dev) for _ in range(2))
+        kv = nat.kv_layout_paged(cache, cache, torch.zeros(B, 1, dtype=torch.int32, device=dev))
+        idx, count = torch.zeros(B, G, 4, dtype=torch.int32, device=dev), torch.zeros(B, G, dtype=torch.int32, device=dev)
+        if entry == "sparse":
+            nat.decode_sparse_paged(q, kv, idx, count, 4, None, 1.0, out, None, None, 1)
+        elif entry == "noalloc":
+            nat.decode_sparse_paged_noalloc(q, kv, idx, count, 4, None, 1.0, out, None, 1)
+        else:
+            logits, pooled = torch.zeros(B, H, 4, device=dev), torch.zeros(B, G, 4, device=dev)
+            nat.decode_anchor_paged(q, kv, count.view(B), 4, 1.0, logits, pooled, out, torch.zeros(B, H, device=dev), None, 1)
+
+    with pytest.raises(nat.KascadeNativeError) as refused:
+        call(65536)
+    assert (torch.ones(64, device=dev) + 1).sum().item() == 128          # PyTorch checks the last error after its launch
+    call(2)
+    torch.cuda.synchronize()
+    assert "decode_attn_kernel" in str(refused.value)
