@@ -68,7 +68,9 @@ constexpr float kLog2e = 1.4426950408889634f;
 // Programmatic dependent launch.  Every kernel of the attention path starts with pdl_begin(): it waits until the kernel
 // before it in the stream has completed and its writes are visible, then lets the kernel after it be set up.  That
 // one's launch, block scheduling and parameter loads so fall into this one's run time instead of a gap of 1.5-2 us
-// after it.  Nothing may touch global memory before the wait.
+// after it.  Nothing may touch global memory before the wait, and nothing may be read through the non-coherent path
+// (__ldg, ld.global.nc, a `const T* __restrict__` parameter): that asks for memory which nobody writes while the kernel
+// lives, and this kernel lives already while the one before it writes its inputs.
 __device__ __forceinline__ void pdl_begin() {
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");

@@ -244,11 +244,11 @@ __global__ void __launch_bounds__(dec_warps(KV) * 32, 1) decode_attn_kernel(cons
     int s = (st_begin + warp + j * WARPS) * kSub + (lane & 15);
     if (j >= my_count) return 0;
     s = min(s, n - 1);
-    return DENSE ? s : __ldg(idx_row + s);
+    return DENSE ? s : idx_row[s];
   };
   auto load_page = [&](int pos) -> int {
     int lp = pos >> p.page_shift;
-    return table ? __ldg(table + lp) : lp;
+    return table ? table[lp] : lp;
   };
   auto issue = [&](int j, int pos, int page) {
     if (j < my_count) {
@@ -285,8 +285,8 @@ __global__ void __launch_bounds__(dec_warps(KV) * 32, 1) decode_attn_kernel(cons
   auto load_scale = [&](int page, float& sk, float& sv) {
     if (FP8) {
       const int64_t at = sc_base + (int64_t)page * p.sc_stride_page;
-      sk = __ldg(p.k_scale + at);
-      sv = HAS_V ? __ldg(p.v_scale + at) : 1.f;
+      sk = p.k_scale[at];
+      sv = HAS_V ? p.v_scale[at] : 1.f;
     }
   };
 
@@ -485,9 +485,8 @@ __global__ void __launch_bounds__(dec_warps(KV) * 32, 1) decode_attn_kernel(cons
 // come from shuffles, and the partial outputs are loaded eight at a time (one after the other they took 4.5 us for 18
 // splits, against 2.9 us).
 template <bool HAS_V, bool BF16>
-__global__ void __launch_bounds__(kD) decode_combine_kernel(const float* __restrict__ ws_m,
-                                                            const float* __restrict__ ws_l,
-                                                            const float* __restrict__ ws_o,
+__global__ void __launch_bounds__(kD) decode_combine_kernel(const float* ws_m, const float* ws_l,
+                                                            const float* ws_o,
                                                             __half* __restrict__ out,
                                                             float* __restrict__ lse2, int H,
                                                             int num_splits) {
@@ -531,9 +530,8 @@ __global__ void __launch_bounds__(kD) decode_combine_kernel(const float* __restr
 }
 
 // pooled[b,g,j] = sum_h exp2(logit[b,4g+h,j] - lse2[b,4g+h]); grid (ceil(maxlen/1024), G, B)
-__global__ void __launch_bounds__(256) decode_pool_kernel(const float* __restrict__ logits,
-                                                          const float* __restrict__ lse2,
-                                                          const int32_t* __restrict__ seq_lens,
+__global__ void __launch_bounds__(256) decode_pool_kernel(const float* logits, const float* lse2,
+                                                          const int32_t* seq_lens,
                                                           float* __restrict__ pooled,
                                                           int64_t stride, int H, int G) {
   pdl_begin();

@@ -388,7 +388,7 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
     auto key_of = [&](const GatherTile& g, int j, int r) -> int {
       const int s = j * 128 + r_begin + r * 32 + lane;
       if (s >= g.total || (r == 1 && (!has_tail || lane >= 16))) return 0;
-      return s < g.count ? __ldg(g.idx + s) : g.tile_start + (s - g.count);
+      return s < g.count ? g.idx[s] : g.tile_start + (s - g.count);
     };
     GatherTile cur = fetch(0);
     int a0 = 0, a1 = 0, b0 = 0, b1 = 0;                  // keys of the next block and of the one after it

@@ -158,8 +158,8 @@ __device__ __forceinline__ int decode_budget(const DecodeBudget& d, int n) {
 
 template <int C, int kTopkWarps>       // CTAs that share a row (a cluster of C), warps per CTA
 __global__ void __launch_bounds__(kTopkWarps * 32, 32 / kTopkWarps)
-topk_select_kernel(const float* __restrict__ scores, int64_t row_stride, int n_cols,
-                   const int32_t* __restrict__ n_valid, const int32_t* __restrict__ k_row, int k_max,
+topk_select_kernel(const float* scores, int64_t row_stride, int n_cols,
+                   const int32_t* n_valid, const int32_t* k_row, int k_max,
                    int32_t* __restrict__ out_idx, int64_t idx_stride, int32_t* __restrict__ out_count,
                    int64_t rows, const DecodeBudget budget) {
   namespace cg = cooperative_groups;
@@ -212,7 +212,7 @@ topk_select_kernel(const float* __restrict__ scores, int64_t row_stride, int n_c
       for (int it = 0; it < kMaxF4; ++it) {
         if (it < f4) {
           const int pos = (int)(((int64_t)(it * kTopkThreads + tid) * n4) >> (f4 == kF4 ? 10 : 11));  // < n4 - 1
-          const float4 x = __ldg(row4 + pos);
+          const float4 x = row4[pos];
           sk[it * 4 + 0] = float_key(x.x); sk[it * 4 + 1] = float_key(x.y);
           sk[it * 4 + 2] = float_key(x.z); sk[it * 4 + 3] = float_key(x.w);
         } else {
@@ -314,7 +314,7 @@ topk_select_kernel(const float* __restrict__ scores, int64_t row_stride, int n_c
 #pragma unroll
         for (int j = 0; j < kTopkUnroll; ++j) {
           const int i4 = w_begin + (it0 + j) * 32 + lane;
-          xs[j] = i4 < w_end ? __ldg(row4 + i4) : make_float4(0.f, 0.f, 0.f, 0.f);
+          xs[j] = i4 < w_end ? row4[i4] : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
         for (int j = 0; j < kTopkUnroll; ++j) {
@@ -473,7 +473,7 @@ topk_select_kernel(const float* __restrict__ scores, int64_t row_stride, int n_c
         __syncthreads();
         for (int it = 0; it < iters; ++it) {
           const int i4 = it * kTopkThreads + tid;
-          const float4 x = i4 < n4 ? __ldg(row4 + i4) : make_float4(0.f, 0.f, 0.f, 0.f);
+          const float4 x = i4 < n4 ? row4[i4] : make_float4(0.f, 0.f, 0.f, 0.f);
           uint32_t u[4];
           piece_keys(x, i4 < n4 ? i4 : n4, n4, n, u);
 #pragma unroll
@@ -501,7 +501,7 @@ topk_select_kernel(const float* __restrict__ scores, int64_t row_stride, int n_c
   #pragma unroll
           for (int j = 0; j < kTopkUnroll; ++j) {
             const int i4 = w_begin + (it0 + j) * 32 + lane;
-            xs[j] = i4 < w_end ? __ldg(row4 + i4) : make_float4(0.f, 0.f, 0.f, 0.f);
+            xs[j] = i4 < w_end ? row4[i4] : make_float4(0.f, 0.f, 0.f, 0.f);
           }
   #pragma unroll
           for (int j = 0; j < kTopkUnroll; ++j) {
@@ -556,7 +556,7 @@ topk_select_kernel(const float* __restrict__ scores, int64_t row_stride, int n_c
 #pragma unroll
       for (int j = 0; j < kTopkUnroll; ++j) {
         const int i4 = w_begin + (it0 + j) * 32 + lane;
-        xs[j] = i4 < w_end ? __ldg(row4 + i4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        xs[j] = i4 < w_end ? row4[i4] : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
       for (int j = 0; j < kTopkUnroll; ++j) {
