@@ -571,12 +571,15 @@ class EfficientKascadeStrategy(Strategy):
                              mean_seq_len: Optional[float] = None) -> torch.Tensor:
         """Paged-attention backend entry: query [B,H,D] fp16 / bf16, key/value cache
         [num_pages, page_size, G, D] of the same type, block_table [B, max_pages] int32, seq_lens [B] int32
-        -> out [B,H,D].  An FP8 (e4m3) cache comes with k_scale / v_scale [num_pages, G] fp32 and takes fp16
-        queries.  `mean_seq_len` is a hint of the host for batches of very different lengths (the work is then cut
-        into more, smaller pieces); results do not depend on it beyond summation order.  The reference has no paged kernel (README.md:135); the nearest
-        signature is kernels/flash_decoding/reuse_kascade_gqa_decode_with_kvcache.py:160-171."""
+        (other integer types are converted) -> out [B,H,D].  An FP8 (e4m3) cache comes with k_scale / v_scale
+        [num_pages, G] fp32 and takes fp16 queries.  `mean_seq_len` is a hint of the host for batches of very different
+        lengths (the work is then cut into more, smaller pieces); results do not depend on it beyond summation order.
+        The reference has no paged kernel (README.md:135); the nearest signature is
+        kernels/flash_decoding/reuse_kascade_gqa_decode_with_kvcache.py:160-171."""
         if max_seq_len is None:
             max_seq_len = int(seq_lens.max().item())
+        if seq_lens.dtype != torch.int32 or not seq_lens.is_contiguous():     # the kernels read contiguous int32
+            seq_lens = seq_lens.to(torch.int32).contiguous()
         kv = nat.kv_layout_paged(key_cache, value_cache, block_table, k_scale, v_scale)
         return self._decode(int(layer_idx), query, kv, seq_lens, int(max_seq_len), scaling, key_cache.shape[2],
                             mean_len=mean_seq_len)

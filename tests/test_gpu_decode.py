@@ -313,3 +313,26 @@ def test_a_refused_launch_names_its_kernel_and_leaves_no_error_behind(entry):
     call(2)
     torch.cuda.synchronize()
     assert "decode_attn_kernel" in str(refused.value)
+
+
+@pytest.mark.parametrize("form", ["int32", "int64", "int16", "strided"])
+def test_sequence_lengths_of_any_integer_type_and_stride(form):
+    """The paged entry takes seq_lens as the caller holds them; every form gives what contiguous int32 gives."""
+    from kascade_b200 import EfficientKascadeStrategy
+    dev = torch.device("cuda")
+    g = torch.Generator(device="cuda").manual_seed(8)
+    for lens in ([700], [700, 300, 129]):
+        B, G, H, D, page = len(lens), 1, 4, 128, 16
+        pages = -(-max(lens) // page)
+        k, v = (torch.randn(B * pages, page, G, D, generator=g, device=dev).half() for _ in range(2))
+        table = torch.arange(B * pages, dtype=torch.int32, device=dev).view(B, pages)
+        q = torch.randn(B, H, D, generator=g, device=dev).half()
+        n = torch.tensor(lens, dtype=torch.int32, device=dev)
+        given = {"int32": n, "int64": n.long(), "int16": n.short(), "strided": torch.stack([n, n + 5], 1)[:, 0]}[form]
+
+        def step(seq_lens):
+            s = EfficientKascadeStrategy([0], "x/y", k=20, tile_size=32, head_mapping=[[0]] * 2, register=False)
+            return [s.paged_decode_forward(l, q, k, v, table, seq_lens, D ** -0.5, max_seq_len=max(lens)) for l in range(2)]
+
+        for layer, (got, want) in enumerate(zip(step(given), step(n))):
+            assert torch.equal(got, want), f"layer {layer}, {lens}"
