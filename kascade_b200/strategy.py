@@ -312,7 +312,10 @@ class EfficientKascadeStrategy(Strategy):
 
     def _pad_bounds(self, pad, dev):
         """(first rows, lengths) of a padded batch on the device and its lengths on the host; copied once per mask, not
-        once per layer."""
+        once per layer.  Not under capture: a graph would keep the addresses of tensors that the next mask replaces."""
+        if torch.cuda.is_current_stream_capturing():
+            raise nat.KascadeNativeError("a padded prompt cannot be captured into a CUDA graph: its rows and lengths are "
+                                         "copied from the host")
         cached = getattr(self, "_pad_dev", None)
         if cached is None or cached[0] is not pad or cached[1].device != dev:
             both = torch.tensor(pad, dtype=torch.int32, device=dev)

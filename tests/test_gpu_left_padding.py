@@ -138,3 +138,36 @@ def test_zero_padding_clears_exactly_the_rows_outside(L, dtype):
             s = 0 if first is None else first[b]
             inside = (pos >= s) & (pos < s + n)
             assert bool((out[b].cpu()[inside] == 7).all()) and bool((out[b].cpu()[~inside] == 0).all()), (L, b)
+
+
+def _small_strategy():
+    from kascade_b200 import EfficientKascadeStrategy
+    return EfficientKascadeStrategy([0], "x/y", k=20, tile_size=32, head_mapping=[[0, 1], [1, 0]], register=False)
+
+
+def _layer(index):
+    class M:
+        num_key_value_groups = 4
+        layer_idx = index
+    return M()
+
+
+@pytest.mark.filterwarnings("ignore:The CUDA Graph is empty")
+def test_a_padded_prompt_is_refused_under_capture():
+    """A padded prompt's rows and lengths are copied from the host, so a graph would hold the addresses of tensors that the
+    next mask replaces: capturing it is refused, also when the mask has been seen before, and the strategy stays usable."""
+    from kascade_b200 import _native as nat
+    dev = torch.device("cuda")
+    g = torch.Generator(device="cuda").manual_seed(2)
+    B, H, G, D, L = 2, 8, 2, 128, 200
+    q = torch.randn(B, H, L, D, generator=g, device=dev).half()
+    k, v = (torch.randn(B, G, L, D, generator=g, device=dev).half() for _ in range(2))
+    s, mask = _small_strategy(), _mask([0, 37], L, L)
+    want = [s.attention_forward(_layer(l), q, k, v, mask, D ** -0.5)[0] for l in range(2)]
+    torch.cuda.synchronize()
+    for l in range(2):
+        with pytest.raises(nat.KascadeNativeError, match="capture"):
+            with torch.cuda.graph(torch.cuda.CUDAGraph()):
+                s.attention_forward(_layer(l), q, k, v, mask, D ** -0.5)
+    for l in range(2):
+        assert torch.equal(s.attention_forward(_layer(l), q, k, v, mask, D ** -0.5)[0], want[l])
