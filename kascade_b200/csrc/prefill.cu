@@ -1280,9 +1280,10 @@ selftest_wait_timeout_kernel(int32_t* __restrict__ result, unsigned long long li
 constexpr int kPadRows = 8;
 __global__ void __launch_bounds__(256) zero_padding_kernel(uint4* __restrict__ out, const int32_t* __restrict__ seq_start,
                                                            const int32_t* __restrict__ seq_len, int max_len, int row16) {
-  const int b = blockIdx.y;
+  const int groups = (max_len + kPadRows - 1) / kPadRows;              // CTAs per slot; all slots along x, which holds any batch
+  const int b = blockIdx.x / groups;
   const int begin = seq_start ? seq_start[b] : 0, end = begin + max(seq_len[b], 0);
-  const int r0 = blockIdx.x * kPadRows, r1 = min(r0 + kPadRows, max_len);
+  const int r0 = (blockIdx.x - b * groups) * kPadRows, r1 = min(r0 + kPadRows, max_len);
   if (r0 >= begin && r1 <= end) return;
   for (int r = r0; r < r1; ++r) {
     if (r >= begin && r < end) continue;
@@ -1689,12 +1690,14 @@ extern "C" int kb200_zero_padding(void* out, const kb200_ragged* ragged, int bat
   using namespace kb200;
   KB_ENTRY(out, "zero_padding: out");
   KB_REQUIRE(out && ragged && ragged->seq_len, "zero_padding: null pointer");
-  KB_REQUIRE(batch >= 0 && batch <= 65535 && max_len >= 0, "zero_padding: batch %d, %d rows", batch, max_len);
+  KB_REQUIRE(batch >= 0 && max_len >= 0, "zero_padding: negative size");
   KB_REQUIRE(row_bytes > 0 && row_bytes % 16 == 0 && row_bytes / 16 < (1ll << 30) &&
                  (reinterpret_cast<uintptr_t>(out) & 15) == 0,
              "zero_padding: rows must be 16-byte aligned");
   if (batch == 0 || max_len == 0) return 0;
-  zero_padding_kernel<<<dim3(ceil_div(max_len, kPadRows), batch), 256, 0, (cudaStream_t)stream>>>(
+  const int64_t ctas = (int64_t)batch * ceil_div(max_len, kPadRows);
+  KB_REQUIRE(ctas < (1ll << 31), "zero_padding: too many rows");
+  zero_padding_kernel<<<(unsigned)ctas, 256, 0, (cudaStream_t)stream>>>(
       static_cast<uint4*>(out), ragged->seq_start, ragged->seq_len, max_len, (int)(row_bytes / 16));
   KB_CHECK_LAUNCH("zero_padding_kernel");
   return 0;

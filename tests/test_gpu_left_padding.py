@@ -171,3 +171,14 @@ def test_a_padded_prompt_is_refused_under_capture():
                 s.attention_forward(_layer(l), q, k, v, mask, D ** -0.5)
     for l in range(2):
         assert torch.equal(s.attention_forward(_layer(l), q, k, v, mask, D ** -0.5)[0], want[l])
+
+
+def test_zero_padding_of_more_sequences_than_a_grid_row_holds():
+    from kascade_b200 import _native as nat
+    dev = torch.device("cuda")
+    B, L = 65537, 3
+    lens = torch.arange(B, dtype=torch.int32, device=dev) % (L + 1)
+    out = torch.ones(B, L, 8, dtype=torch.float16, device=dev)
+    nat.zero_padding(out, nat.ragged(None, lens))
+    inside = torch.arange(L, device=dev)[None, :] < lens[:, None]
+    assert torch.equal(out, inside[:, :, None].expand(B, L, 8).half())
