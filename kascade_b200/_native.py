@@ -94,7 +94,10 @@ class PushPlan(C.Structure):
 
 _lib = None
 _inited = set()
-launch_count = 0          # kernels of this library launched so far by this process (host-side tally)
+# Host-side tallies of the kernels of this library launched so far by this process: those that compute, and those that
+# clear the padding of a ragged batch's output, one per padded prompt layer, which stand for a memset.
+launch_count = 0
+clear_count = 0
 
 
 def _launched(n: int):
@@ -495,13 +498,15 @@ def prefill_dense(q, k, v, scale, out, lse2, fanout: Optional[OutFanout] = None,
 @_on_device_of(0)
 def zero_padding(out: torch.Tensor, ragged: Ragged):
     """Zeros the rows of out [B, L, ...] (contiguous) that lie outside the sequences."""
+    global clear_count
     lib = init(out.get_device())
     assert out.is_contiguous()
     B, L = out.shape[:2]
     if out.numel() == 0:
         return
     _check(lib.kb200_zero_padding(_ptr(out), C.byref(ragged), B, L, out.numel() * out.element_size() // (B * L), _stream()),
-           "kb200_zero_padding")                     # (stands for a memset: not in launch_count)
+           "kb200_zero_padding")
+    clear_count += 1
 
 
 @_on_device_of(0)

@@ -182,3 +182,22 @@ def test_zero_padding_of_more_sequences_than_a_grid_row_holds():
     nat.zero_padding(out, nat.ragged(None, lens))
     inside = torch.arange(L, device=dev)[None, :] < lens[:, None]
     assert torch.equal(out, inside[:, :, None].expand(B, L, 8).half())
+
+
+def test_the_clear_of_a_padded_layer_is_tallied():
+    """Every kernel of a padded prompt's layer is in a tally: the computing ones in launch_count, the clear of the padding in
+    clear_count; an unpadded layer and an empty output clear nothing."""
+    from kascade_b200 import _native as nat
+    dev = torch.device("cuda")
+    B, H, G, D, L = 2, 8, 2, 128, 200
+    q = torch.zeros(B, H, L, D, dtype=torch.float16, device=dev)
+    k = torch.zeros(B, G, L, D, dtype=torch.float16, device=dev)
+    s = _small_strategy()
+    for mask, clears in ((_mask([0, 37], L, L), 1), (None, 0)):
+        for l, launches in ((0, 4), (1, 1)):
+            before = nat.launch_count, nat.clear_count
+            s.attention_forward(_layer(l), q, k, k, mask, 1.0)
+            assert (nat.launch_count - before[0], nat.clear_count - before[1]) == (launches, clears), (l, clears)
+    before = nat.clear_count
+    nat.zero_padding(q.new_empty(0, L, D), nat.ragged(None, torch.zeros(1, dtype=torch.int32, device=dev)))
+    assert nat.clear_count == before
