@@ -201,3 +201,22 @@ def test_the_clear_of_a_padded_layer_is_tallied():
     before = nat.clear_count
     nat.zero_padding(q.new_empty(0, L, D), nat.ragged(None, torch.zeros(1, dtype=torch.int32, device=dev)))
     assert nat.clear_count == before
+
+
+def test_one_strategy_sees_a_second_mask_and_an_edited_one():
+    """Rows and lengths are copied to the device once per mask: another mask, and the same one edited in place, replace them."""
+    dev = torch.device("cuda")
+    g = torch.Generator(device="cuda").manual_seed(3)
+    B, H, G, D, L = 3, 8, 2, 128, 300
+    q = torch.randn(B, H, L, D, generator=g, device=dev).half()
+    k, v = (torch.randn(B, G, L, D, generator=g, device=dev).half() for _ in range(2))
+    s = _small_strategy()
+    first, second = _mask([0, 40, 90], L, L), _mask([33, 0, 5], L, L, right=[0, 9, 0])
+    for turn, mask in enumerate([first, second, second, first]):
+        if turn == 2:
+            mask.copy_(_mask([150, 1, 0], L, L))
+        alone = _small_strategy()
+        for l in range(2):
+            got = s.attention_forward(_layer(l), q, k, v, mask, D ** -0.5)[0]
+            want = alone.attention_forward(_layer(l), q, k, v, mask.clone(), D ** -0.5)[0]
+            assert torch.equal(got, want), f"mask {turn}, layer {l}"

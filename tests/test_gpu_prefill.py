@@ -241,8 +241,8 @@ def test_rejected_arguments_name_the_problem():
 @pytest.mark.parametrize("L", [1, 31, 33, 128, 129, 160, 385, 513, 640, 1025])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_lse_and_pooled_scores_at_the_edges_of_the_streams(L, dtype):
-    """The passes without V deal key blocks of 128 to three (lse) and four (pool) streams and keep two Q tiles: prompts of
-    1 to 9 blocks, full and ragged last blocks, against 64 bits.  Products are exact in fp32, a row's 128 to 1025 terms and
+    """The passes without V deal key blocks of 128 to three (lse) and four (pool) streams: prompts of 1 to 9
+    blocks, full and ragged last blocks, a tile to each CTA, against 64 bits.  Products are exact in fp32, a row's 128 to 1025 terms and
     their polynomial exponentials (3e-6) add up to well under 2e-5; pooled scores are sums of such terms."""
     from kascade_b200 import _native as nat
     dev = torch.device("cuda")
@@ -267,4 +267,42 @@ def test_lse_and_pooled_scores_at_the_edges_of_the_streams(L, dtype):
         if start:
             assert ((pooled[:, :, t, :start].double() - ref).abs() / ref.clamp_min(1e-6)).max().item() < 5e-5, t
         assert bool((pooled[:, :, t, start:] == -7.0).all()), "entries from the tile on are not written"
+    assert nat.read_status() == 0
+
+
+@pytest.mark.parametrize("L", [577, 1025])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("ragged", [False, True], ids=["full", "ragged"])
+def test_lse_and_pooled_scores_over_several_tiles_of_a_cta(L, dtype, ragged):
+    """608 and 1056 tiles on 148 SMs: every CTA goes through four to eight of them, so both Q tiles, the look-ahead into the next
+    tile and the block numbers that run on across tiles are in use.  Ragged: an empty sequence and one of a single tile lie
+    between the others, so that tiles without blocks fall between those with some.  Bounds as in the test above."""
+    from kascade_b200 import _native as nat
+    dev = torch.device("cuda")
+    g = torch.Generator().manual_seed(L)
+    B, H, G, D, tile = 4, 32, 8, 128, 32
+    lens, starts = ([L, 0, 32, L - 200], [0, 5, L - 32, 100]) if ragged else ([L] * B, [0] * B)
+    q = torch.randn(B, L, H, D, generator=g).to(dtype).to(dev)
+    k = torch.randn(B, L, G, D, generator=g).to(dtype).to(dev)
+    T, scale = -(-L // tile), 0.6 * D ** -0.5
+    at = torch.tensor([starts, lens], dtype=torch.int32, device=dev)
+    rg = nat.ragged(at[0], at[1]) if ragged else None
+    lse2 = torch.full((B, L, H), -7.0, device=dev)
+    pooled = torch.full((B, G, T, -(-L // 128) * 128), -7.0, device=dev)
+    nat.prefill_dense(q, k, None, scale, None, lse2, ragged=rg)
+    nat.prefill_pool_scores(q, k, lse2, scale, pooled, ragged=rg)
+    for b, n in enumerate(lens):
+        qb, kb = (x[b, starts[b]:starts[b] + n].double() for x in (q, k))
+        s = torch.einsum("ighd,jgd->ghij", qb.view(n, G, 4, D), kb) * scale
+        s = s.masked_fill(~torch.ones(n, n, dtype=torch.bool, device=dev).tril(), float("-inf"))
+        if n:
+            got = lse2[b, :n].double().view(n, G, 4).permute(1, 2, 0) * 0.6931471805599453
+            assert (got - torch.logsumexp(s, -1)).abs().max().item() < 2e-5, b
+        p = torch.softmax(s, -1).sum(1)                               # [G, i, j]
+        for t in range(T):
+            start = t * tile if t * tile < n else 0
+            ref = p[:, start:start + tile, :start].sum(1)
+            if start:
+                assert ((pooled[b, :, t, :start].double() - ref).abs() / ref.clamp_min(1e-6)).max().item() < 5e-5, (b, t)
+            assert bool((pooled[b, :, t, start:] == -7.0).all()), "entries from the tile on are not written"
     assert nat.read_status() == 0

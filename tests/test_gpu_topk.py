@@ -173,14 +173,14 @@ def test_decode_selection_rejects_bad_arguments():
 
 @pytest.mark.parametrize("rows,n", [(1, 8191), (1, 8192), (1, 16384), (3, 32768), (8, 131071), (37, 33000), (38, 33000), (74, 16400),
                                     (75, 16400), (148, 16400), (149, 16400), (444, 700), (444, 3001), (444, 8192), (444, 8193),
-                                    (444, 40001)])
+                                    (444, 40001), (75, 70001), (200, 65537), (444, 65537), (444, 100003)])
 @pytest.mark.parametrize("kind", ["smooth", "ties", "steps"])
 def test_any_number_of_threads_selects_the_same(rows, n, kind):
     """Few long rows are split over the CTAs of a cluster (2, 4 or 8, by rows and columns), many rows get CTAs of 4 or 8
-    warps each.  The selection is exact, so it
-    equals a stable sort's, ties from the lowest index, whatever the number of CTAs: also where the sample's bracket
-    fails (`ties`: half of the row has one value; `steps`: four values) and where single rows are short, empty or
-    selected as a whole."""
+    warps each, and rows of more than 65536 scores a sample of twice the size, in clusters and out of them.  The selection
+    is exact, so it equals a stable sort's, ties from the lowest index, whatever the number of CTAs: also where the
+    sample's bracket fails (`ties`: half of the row has one value; `steps`: four values) and where single rows are
+    short, empty or selected as a whole."""
     from kascade_b200 import _native as nat
     dev = torch.device("cuda")
     g = torch.Generator().manual_seed(rows * 7 + n)
@@ -209,3 +209,34 @@ def test_any_number_of_threads_selects_the_same(rows, n, kind):
             want = torch.sort(scores[r, :m], descending=True, stable=True).indices[:k].sort().values
         assert torch.equal(out[r, :k].long(), want), f"row {r}"
         assert (out[r, k:] == -7).all()
+
+
+@pytest.mark.parametrize("warps,n_cols", [(8, 8193), (4, 4500)])
+def test_a_cta_selects_from_one_kind_of_row_after_another(warps, n_cols):
+    """More rows than the grid holds (1024 threads' worth of CTAs of 4 or 8 warps for each of 32 waves): the first CTAs take a
+    second row, with the shared lists and histogram of the first.  Rows are empty, whole, tied, short or long enough to
+    be sampled, in an order that puts every kind after another one."""
+    from kascade_b200 import _native as nat
+    dev = torch.device("cuda")
+    grid = nat.sm_count(0) * 1024 // warps
+    rows = grid + 512
+    stride = -(-n_cols // 4) * 4
+    scores = torch.rand(rows, stride, generator=torch.Generator(device="cuda").manual_seed(n_cols), device=dev) ** 6
+    kind = torch.arange(rows, device=dev) % 5
+    scores[kind == 2] = 0.5
+    n_valid = torch.tensor([0, 700, 900, 1200, n_cols], dtype=torch.int32, device=dev)[kind]
+    k_row = torch.tensor([128, 700, 130, 128, n_cols // 10], dtype=torch.int32, device=dev)[kind]
+    k_max = 900
+    out = torch.full((rows, k_max), -7, dtype=torch.int32, device=dev)
+    cnt = torch.full((rows,), -1, dtype=torch.int32, device=dev)
+    nat.topk_select(scores, n_valid, k_row, k_max, out, cnt, n_cols=n_cols)
+    k = torch.minimum(n_valid, k_row)
+    assert torch.equal(cnt, k)
+    twice = torch.cat([torch.arange(rows - grid, device=dev), torch.arange(grid, rows, device=dev)])     # a CTA's two rows
+    pos = torch.arange(n_cols, device=dev)
+    masked = scores[twice, :n_cols].masked_fill(pos[None, :] >= n_valid[twice, None], -1.0)
+    want = torch.sort(masked, dim=-1, descending=True, stable=True).indices[:, :k_max]
+    taken = torch.arange(k_max, device=dev)[None, :] < k[twice, None]
+    want = torch.sort(want.masked_fill(~taken, n_cols), dim=-1).values
+    assert torch.equal(out[twice].masked_fill(~taken, n_cols).long(), want)
+    assert bool((out[twice][~taken] == -7).all())
