@@ -188,7 +188,7 @@ __device__ __forceinline__ int longest_first(int r, int n, const Len& len) {
 // partial until the end.
 template <bool DENSE, bool HAS_V, bool WRITE_LOGITS, int KV>
 __global__ void __launch_bounds__(dec_warps(KV) * 32, 1) decode_attn_kernel(const DecodeParams p) {
-  pdl_begin();
+  pdl_wait();
   constexpr bool BF16 = KV == 1, FP8 = KV == 2;
   const int WARPS = blockDim.x >> 5;       // dec_warps(KV) or half of it, chosen at launch
   constexpr uint32_t FULL = 0xFFFFFFFFu;
@@ -430,6 +430,7 @@ __global__ void __launch_bounds__(dec_warps(KV) * 32, 1) decode_attn_kernel(cons
   }
   cp_async_wait<0>();
   __syncthreads();
+  pdl_trigger();                       // only the merge is left: most SMs have room by now
 
   // ---- merge the warps of this CTA through shared memory ------------------------------------------
 #pragma unroll
@@ -534,7 +535,7 @@ __global__ void __launch_bounds__(256) decode_pool_kernel(const float* logits, c
                                                           const int32_t* seq_lens,
                                                           float* __restrict__ pooled,
                                                           int64_t stride, int H, int G) {
-  pdl_begin();
+  pdl_wait();                          // (no trigger: the next kernel is set up as these CTAs end)
   const int b = blockIdx.z, g = blockIdx.y;
   const int n = seq_lens[b];
   const int j = (blockIdx.x * 256 + threadIdx.x) * 4;

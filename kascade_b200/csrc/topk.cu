@@ -169,7 +169,7 @@ topk_select_kernel(const float* scores, int64_t row_stride, int n_cols,
   extern __shared__ uint32_t merged[];                    // C > 1: the lists of all CTAs of the cluster
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int rank = C > 1 ? (int)cg::this_cluster().block_rank() : 0;
-  pdl_begin();
+  pdl_wait();
 
   for (int64_t row = blockIdx.x / C; row < rows; row += gridDim.x / C) {
     int n, k;
@@ -550,6 +550,7 @@ topk_select_kernel(const float* scores, int64_t row_stride, int n_cols,
         eq_before += peer->cta_equal;
       }
     }
+    if (row + gridDim.x / C >= rows) pdl_trigger();       // the CTA's last row, and its last pass
     // ---- 4. write the selected positions of this warp's piece, in index order -----------------------------
     for (int it0 = 0; it0 < w_iters; it0 += kTopkUnroll) {
       float4 xs[kTopkUnroll];

@@ -151,16 +151,17 @@ def test_layout_helpers_refuse_host_tensors():
 
 
 def test_kernels_that_start_early_use_no_non_coherent_loads():
-    """A kernel with pdl_begin() is resident while the kernel before it may still write its inputs.  The non-coherent load
-    (__ldg, ld.global.nc, and what the compiler makes of a `const T* __restrict__` parameter) is defined only for memory
-    that nothing writes while the kernel lives, so such a kernel has none, nor has a function of its file that it may call."""
+    """A kernel with pdl_wait() or pdl_begin() is resident while the kernel before it may still write its inputs.  The
+    non-coherent load (__ldg, ld.global.nc, and what the compiler makes of a `const T* __restrict__` parameter) is defined
+    only for memory that nothing writes while the kernel lives, so such a kernel has none, nor has a function of its file
+    that it may call."""
     csrc = os.path.join(ROOT, "kascade_b200", "csrc")
     early = 0
     for name in sorted(os.listdir(csrc)):
         text = re.sub(r"//[^\n]*|/\*.*?\*/", "", open(os.path.join(csrc, name)).read(), flags=re.S)
         heads = list(re.finditer(r"__global__[^;{]*?\b(\w+)\s*\(([^{;]*)\)\s*\{", text))
         ends = [m.start() for m in heads[1:]] + [len(text)]
-        pdl = [m for m, end in zip(heads, ends) if "pdl_begin();" in text[m.end():end]]
+        pdl = [m for m, end in zip(heads, ends) if re.search(r"\bpdl_(wait|begin)\(\);", text[m.end():end])]
         early += len(pdl)
         for m in pdl:
             assert not re.search(r"const[^,]*__restrict__", m.group(2)), f"{name}: {m.group(1)} has a const __restrict__ parameter"
