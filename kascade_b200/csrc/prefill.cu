@@ -6,7 +6,7 @@
 //
 //   kDenseAttn  causal attention over keys 0 .. last query of the tile; writes O and lse2
 //               (replaces `prefill`, kernels/flash_attention/recompute_kascade_gqa_prefill.py:224-274)
-//   kDenseLse   the same without V: lse2 only
+//   kDenseLse   the same without V: lse2 only (kShortLse: the same for short prompts, see kShortLseRows)
 //               (replaces `compute_scores`, recompute_kascade_gqa_prefill.py:276-312)
 //   kSparse     keys = the tile's selected index row followed by the tile's own keys
 //               (replaces `main_kernel`, kernels/flash_attention/reuse_kascade_gqa_prefill.py:146-198)
@@ -50,7 +50,7 @@
 
 namespace kb200 {
 
-enum PrefillMode { kDenseAttn = 0, kDenseLse = 1, kSparse = 2, kPool = 3 };
+enum PrefillMode { kDenseAttn = 0, kDenseLse = 1, kSparse = 2, kPool = 3, kShortLse = 4 };
 
 constexpr int kStageBytes = 128 * kD * 2;     // one 128-row operand tile (32 KB)
 constexpr int kNKMax = 4;                     // K ring: 3 stages with a V ring, 4 without
@@ -150,6 +150,18 @@ __device__ __forceinline__ uint64_t ex2_fma2(uint64_t x2) {
   unpair_f(q, q0, q1);
   unpair_f(t, t0, t1);
   return pair_u(__float_as_uint(q0) + (__float_as_uint(t0) << 23), __float_as_uint(q1) + (__float_as_uint(t1) << 23));
+}
+// the same of one value, to the same bits (kShortLse)
+__device__ __forceinline__ float ex2_fma(float x) {
+  x = fmaxf(x, -120.0f);
+  const float t = x + 12582912.0f;
+  const float f = x - (t - 12582912.0f);
+  float q = 0.009585312567651272f;
+  q = fmaf(q, f, 0.05590597912669182f);
+  q = fmaf(q, f, 0.24024048447608948f);
+  q = fmaf(q, f, 0.6931242942810059f);
+  q = fmaf(q, f, 1.0f);
+  return __uint_as_float(__float_as_uint(q) + (__float_as_uint(t) << 23));
 }
 // Which exponentials take that way: of every eight values the fourth and eighth in the lse pass, and the second as
 // well in the pool pass.  The two-element fma occupies the heavy FMA pipe for two cycles, so that pipe (256 + 56 s
@@ -1031,28 +1043,40 @@ tile_prefill_kernel(const __grid_constant__ PrefillParams p, const __grid_consta
         // lse2 = m + log2(l) holds for any reference point m.
         const float m_new = (mx > m_run + kRescaleLog2) ? mx : m_run;
         const float alpha = ex2(m_run - m_new);
-        uint64_t s01 = 0ull, s23 = 0ull;                    // four partial row sums, two per register pair
-        const uint64_t scale_2 = pair_f(p.scale2, p.scale2), nref_2 = pair_f(-m_new, -m_new);
+        float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+        if constexpr (MODE == kShortLse) {
 #pragma unroll
-        for (int part = 0; part < 4; ++part)
+          for (int part = 0; part < 4; ++part)
 #pragma unroll
-          for (int i = 0; i < 32; i += 8) {
-            float x[8], e[8];
-#pragma unroll
-            for (int k2 = 0; k2 < 8; k2 += 2)
-              unpair_f(fma2(pair_u(sr[part][i + k2], sr[part][i + k2 + 1]), scale_2, nref_2), x[k2], x[k2 + 1]);
-            unpair_f(ex2_fma2(pair_f(x[3], x[7])), e[3], e[7]);
-            e[0] = ex2(x[0]); e[1] = ex2(x[1]); e[2] = ex2(x[2]);
-            e[4] = ex2(x[4]); e[5] = ex2(x[5]); e[6] = ex2(x[6]);
-#pragma unroll
-            for (int k2 = 0; k2 < 8; k2 += 4) {
-              s01 = add2(s01, pair_f(e[k2], e[k2 + 1]));
-              s23 = add2(s23, pair_f(e[k2 + 2], e[k2 + 3]));
+            for (int i = 0; i < 32; i += 4) {
+              s0 += ex2(fmaf(__uint_as_float(sr[part][i]), p.scale2, -m_new));
+              s1 += ex2(fmaf(__uint_as_float(sr[part][i + 1]), p.scale2, -m_new));
+              s2 += ex2(fmaf(__uint_as_float(sr[part][i + 2]), p.scale2, -m_new));
+              s3 += ex2_fma(fmaf(__uint_as_float(sr[part][i + 3]), p.scale2, -m_new));
             }
-          }
-        float s0, s1, s2, s3;
-        unpair_f(s01, s0, s1);
-        unpair_f(s23, s2, s3);
+        } else {
+          uint64_t s01 = 0ull, s23 = 0ull;                    // four partial row sums, two per register pair
+          const uint64_t scale_2 = pair_f(p.scale2, p.scale2), nref_2 = pair_f(-m_new, -m_new);
+#pragma unroll
+          for (int part = 0; part < 4; ++part)
+#pragma unroll
+            for (int i = 0; i < 32; i += 8) {
+              float x[8], e[8];
+#pragma unroll
+              for (int k2 = 0; k2 < 8; k2 += 2)
+                unpair_f(fma2(pair_u(sr[part][i + k2], sr[part][i + k2 + 1]), scale_2, nref_2), x[k2], x[k2 + 1]);
+              unpair_f(ex2_fma2(pair_f(x[3], x[7])), e[3], e[7]);
+              e[0] = ex2(x[0]); e[1] = ex2(x[1]); e[2] = ex2(x[2]);
+              e[4] = ex2(x[4]); e[5] = ex2(x[5]); e[6] = ex2(x[6]);
+#pragma unroll
+              for (int k2 = 0; k2 < 8; k2 += 4) {
+                s01 = add2(s01, pair_f(e[k2], e[k2 + 1]));
+                s23 = add2(s23, pair_f(e[k2 + 2], e[k2 + 3]));
+              }
+            }
+          unpair_f(s01, s0, s1);
+          unpair_f(s23, s2, s3);
+        }
         l_run = l_run * alpha + ((s0 + s1) + (s2 + s3));
         m_run = m_new;
       }
@@ -1302,10 +1326,12 @@ int init_prefill() {
   KB_CUDA(cudaFuncSetAttribute(tile_prefill_kernel<kDenseAttn, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemAttn));
   KB_CUDA(cudaFuncSetAttribute(tile_prefill_kernel<kSparse, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemAttn));
   KB_CUDA(cudaFuncSetAttribute(tile_prefill_kernel<kDenseLse, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemNoV));
+  KB_CUDA(cudaFuncSetAttribute(tile_prefill_kernel<kShortLse, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemNoV));
   KB_CUDA(cudaFuncSetAttribute(tile_prefill_kernel<kPool, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemNoV));
   KB_CUDA(cudaFuncSetAttribute(tile_prefill_kernel<kDenseAttn, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemAttn));
   KB_CUDA(cudaFuncSetAttribute(tile_prefill_kernel<kSparse, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemAttn));
   KB_CUDA(cudaFuncSetAttribute(tile_prefill_kernel<kDenseLse, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemNoV));
+  KB_CUDA(cudaFuncSetAttribute(tile_prefill_kernel<kShortLse, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemNoV));
   KB_CUDA(cudaFuncSetAttribute(tile_prefill_kernel<kPool, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemNoV));
   if (!g_encode_tiled) {
     void* fn = nullptr;
@@ -1491,6 +1517,14 @@ static int set_ragged(PrefillParams* p, const kb200_ragged* rg, const char* what
   return 0;
 }
 
+// Prompts up to this length take the lse pass with one exponential per instruction.  A tile of few key blocks keeps one
+// or two softmax warpgroups busy at a time, so a thread's chain of dependent operations counts, and the two-element
+// forms have the longer one (half as many partial sums in flight, and spills around the loop); with all three busy
+// their fewer instructions win.  Same additions in the same order: lse2 is equal to the last bit.  Measured, us with
+// one / two elements per instruction: 64 prompts of 129 / 300 tokens 46.8 / 52.5, 97.3 / 108.4, 16 x 400 37.4 / 41.6,
+// 16 x 1000 124 / 131, 1 x 2048 28.9 / 29.5, 4 x 3001 213 / 212, 1 x 5000 138.8 / 134.6, 1 x 16384 1381 / 1285.
+constexpr int kShortLseRows = 2560;
+
 static int prefill_dense_impl(const kb200_act_layout* q, const kb200_act_layout* k, const kb200_act_layout* v,
                               float softmax_scale, void* out, const kb200_out_fanout* fan, float* lse2, int batch,
                               int seq_len, int num_q_heads, int num_kv_heads, void* stream,
@@ -1521,6 +1555,9 @@ static int prefill_dense_impl(const kb200_act_layout* q, const kb200_act_layout*
     rc = launch_pdl(tile_prefill_kernel<kDenseAttn, true>, grid, PfCfg<kDenseAttn>::kThreads, kSmemAttn, (cudaStream_t)stream, 1, p, tq, tk, tv);
   else if (out)
     rc = launch_pdl(tile_prefill_kernel<kDenseAttn, false>, grid, PfCfg<kDenseAttn>::kThreads, kSmemAttn, (cudaStream_t)stream, 1, p, tq, tk, tv);
+  else if (seq_len <= kShortLseRows)
+    rc = launch_pdl(p.bf16 ? tile_prefill_kernel<kShortLse, true> : tile_prefill_kernel<kShortLse, false>, grid,
+                    PfCfg<kShortLse>::kThreads, kSmemNoV, (cudaStream_t)stream, 1, p, tq, tk, tv);
   else if (p.bf16)
     rc = launch_pdl(tile_prefill_kernel<kDenseLse, true>, grid, PfCfg<kDenseLse>::kThreads, kSmemNoV, (cudaStream_t)stream, 1, p, tq, tk, tv);
   else

@@ -306,3 +306,25 @@ def test_lse_and_pooled_scores_over_several_tiles_of_a_cta(L, dtype, ragged):
                 assert ((pooled[b, :, t, :start].double() - ref).abs() / ref.clamp_min(1e-6)).max().item() < 5e-5, (b, t)
             assert bool((pooled[b, :, t, start:] == -7.0).all()), "entries from the tile on are not written"
     assert nat.read_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_lse_of_short_and_long_prompts_is_the_same_to_the_last_bit(dtype):
+    """Prompts up to 2560 tokens take a variant of the lse pass of their own.  A ragged batch goes by its longest slot, so the
+    same sequences run through one variant alone and through the other inside a longer batch; all give the same bits."""
+    from kascade_b200 import _native as nat
+    dev = torch.device("cuda")
+    g = torch.Generator(device="cuda").manual_seed(6)
+    B, L, H, G, D = 4, 2561, 8, 2, 128
+    lens, starts = [L, 1, 700, 2560], [0, 2000, 33, 1]
+    q = torch.randn(B, L, H, D, generator=g, device=dev).to(dtype)
+    k = torch.randn(B, L, G, D, generator=g, device=dev).to(dtype)
+    at = torch.tensor([starts, lens], dtype=torch.int32, device=dev)
+    together = torch.full((B, L, H), -7.0, device=dev)
+    nat.prefill_dense(q, k, None, 0.07, None, together, ragged=nat.ragged(at[0], at[1]))
+    for b, n in enumerate(lens):
+        alone = torch.full((1, n, H), -7.0, device=dev)
+        rows = slice(starts[b], starts[b] + n)
+        nat.prefill_dense(q[b:b + 1, rows], k[b:b + 1, rows], None, 0.07, None, alone)
+        assert torch.equal(together[b, :n], alone[0]), f"{n} tokens"
+    assert nat.read_status() == 0
