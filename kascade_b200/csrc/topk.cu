@@ -679,23 +679,38 @@ namespace kb200 {
 // that, and for rows under 16384, its fixed phases (the sample, the lists) cost more than a shorter piece saves.
 // Measured, us with one CTA / a cluster: 8 rows of 16384 / 32768 / 131072 scores 17.2 / 25.4 / 69.9 -> 15.2 / 18.5 / 27.1,
 // 32 x 65536 41.4 -> 23.7 (29.2 with two CTAs on an SM), 64 x 32768 25.7 -> 21.1; 128 x 16384 17.8 -> 20.3 with two, 8 x 8192
-// 13.3 -> 13.7: not taken.
+// 13.3 -> 13.7: not taken.  A cluster needs places for all its CTAs in one group of SMs, so where the CTAs of clusters of four
+// or eight would fill the chip some share an SM: they leave an eighth of it free, unless four have long rows to share
+// (37 rows of 16384 / 32768 / 65536 / 131072 in clusters of two / four 16.0 / 18.6, 21.1 / 22.7, 31.4 / 30.6, 48.2 / 44.0;
+// 18 of 65536 in four / eight 24.2 / 28.5).
 static int topk_cluster(int64_t rows, int n_cols) {
   int c = 1;
   if (n_cols < 16384) return c;
-  while (c < 8 && rows * (2 * c) <= sm_count() && n_cols / (2 * c) >= 4096) c *= 2;
+  const int sms = sm_count();
+  while (c < 8 && n_cols / (2 * c) >= 4096 &&
+         rows * (2 * c) <= (c == 1 || (c == 2 && n_cols >= 65536) ? sms : sms * 7 / 8))
+    c *= 2;
   return c;
 }
 
 // Warps of a CTA that has a row to itself.  A row's serial phases (some thirty CTA barriers) are what bounds this kernel
-// when there are many rows, so smaller CTAs, of which more are resident at two thousand threads per SM, hide more of
-// them.  Few rows want many warps each, and rows that do not fit the lists of four warps (about 65536 scores) at least
-// eight.  Measured, us with 16 / 8 / 4 warps: 512 prompt rows of up to 2048 scores 18.2 / 12.6 / 12.5, 3008 x 3001 88 / 50 / 40,
-// 2048 x 8192 92 / 63 / 58, 8192 x 32768 626 / 490 / 505, 24576 x 98304 3776 / 3428 / 7405; decode rows 512 x 32768
-// 68 / 61 / 77, 256 x 16000 23 / 25 / 37, 192 x 65536 58 / 73 / 435.
+// when there are many rows, so smaller CTAs, of which more are resident (a thousand threads per SM at 64 registers),
+// hide more of them.  Few rows want many warps each, and rows that do not fit the lists of four warps (about 65536
+// scores) at least eight.  Measured, us with 16 / 8 / 4 warps: 512 prompt rows of up to 2048 scores 18.2 / 12.6 / 12.5,
+// 3008 x 3001 88 / 50 / 40, 2048 x 8192 92 / 63 / 58, 8192 x 32768 626 / 490 / 505, 24576 x 98304 3776 / 3428 / 7405;
+// decode rows 512 x 32768 68 / 61 / 77, 256 x 16000 23 / 25 / 37, 192 x 65536 58 / 73 / 435.
+// The longer the rows, the more of the time is passes over them and the more the last CTAs to end weigh, above all
+// where the rows differ in length: beyond 32768 scores eight warps need rows for several rounds.  us with 16 / 8:
+// 512 rows of up to 65536 / 131072 scores 96 / 101, 161 / 194; 600 equal ones 154 / 171, 278 / 317; 1024 212 / 208, 389 / 392,
+// of up to that many 156 / 159, 261 / 289; 2048 equal ones 406 / 392, 738 / 745.  A second round of a few rows costs as much: 600 x 24000 / 32768 75.5 / 73.9, 91.2 / 95.5,
+// 800 x 32768 107.4 / 104.4.
 static int topk_warps(int64_t rows, int n_cols) {
-  if (rows < 3ll * sm_count()) return 16;
-  return n_cols <= 8192 ? 4 : 8;
+  const int64_t sms = sm_count();
+  if (rows < 3 * sms) return 16;
+  if (n_cols <= 8192) return 4;
+  if (n_cols > 32768 && rows < (n_cols <= 65536 ? 8 : 14) * sms) return 16;
+  if (n_cols > 24576 && rows > 4 * sms && rows <= 5 * sms) return 16;
+  return 8;
 }
 
 int init_topk() {

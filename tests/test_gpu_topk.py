@@ -173,7 +173,8 @@ def test_decode_selection_rejects_bad_arguments():
 
 @pytest.mark.parametrize("rows,n", [(1, 8191), (1, 8192), (1, 16384), (3, 32768), (8, 131071), (37, 33000), (38, 33000), (74, 16400),
                                     (75, 16400), (148, 16400), (149, 16400), (444, 700), (444, 3001), (444, 8192), (444, 8193),
-                                    (444, 40001), (75, 70001), (200, 65537), (444, 65537), (444, 100003)])
+                                    (444, 40001), (75, 70001), (200, 65537), (444, 65537), (444, 100003),
+                                    (18, 65540), (592, 24577), (593, 24577), (741, 24577), (1183, 32772), (1184, 32772)])
 @pytest.mark.parametrize("kind", ["smooth", "ties", "steps"])
 def test_any_number_of_threads_selects_the_same(rows, n, kind):
     """Few long rows are split over the CTAs of a cluster (2, 4 or 8, by rows and columns), many rows get CTAs of 4 or 8
