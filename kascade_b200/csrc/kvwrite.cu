@@ -71,8 +71,9 @@ __device__ __forceinline__ uint2 quantize8(const H2* x, float scale) {
   return make_uint2(w[0], w[1]);
 }
 
-template <bool BF16, bool FP8>
-__global__ void __launch_bounds__(kKvWriteThreads) kv_write_kernel(const KvWriteParams p) {
+// CTAS: CTAs per SM that the registers have to allow (0: left to the compiler); see launch_kv_write
+template <bool BF16, bool FP8, int CTAS>
+__global__ void __launch_bounds__(kKvWriteThreads, CTAS) kv_write_kernel(const KvWriteParams p) {
   using H2 = typename Pair<BF16>::T;
   using H1 = typename Pair<BF16>::S;
   __shared__ __align__(16) H1 cos_s[kD / 2];
@@ -177,6 +178,19 @@ __global__ void __launch_bounds__(kKvWriteThreads) kv_write_kernel(const KvWrite
   }
 }
 
+// The rows loaded one step ahead take nine registers a thread, which is one resident CTA per SM less.  Where a warp has one
+// step only (24 heads or fewer: appends without Q) nothing is there to load ahead, and with more CTAs than the SMs
+// hold the missing CTA costs time: those are compiled for seven per SM.  Measured before the loads ahead / with them /
+// as it is now, us without Q, with and without rotary table: 32768 tokens 61.0 / 66.5 / 58.3, 56.0 / 63.2 / 54.3; 16 x 600
+// 20.7 / 22.0 / 19.2, 19.2 / 21.2 / 18.2; 64 tokens 2.45 / 2.51 / 2.51, 2.26 / 2.26 / 2.26.
+template <bool BF16, bool FP8>
+static void launch_kv_write(const KvWriteParams& p, int64_t blocks, cudaStream_t st) {
+  if (p.H + 2 * p.G <= kKvWriteThreads / 32 * 4 && blocks > 6ll * sm_count())
+    kv_write_kernel<BF16, FP8, 7><<<(unsigned)blocks, kKvWriteThreads, 0, st>>>(p);
+  else
+    kv_write_kernel<BF16, FP8, 0><<<(unsigned)blocks, kKvWriteThreads, 0, st>>>(p);
+}
+
 }  // namespace kb200
 
 extern "C" int kb200_kv_write(const kb200_act_layout* q_in, void* q_out, const kb200_act_layout* k_new,
@@ -247,10 +261,10 @@ extern "C" int kb200_kv_write(const kb200_act_layout* q_in, void* q_out, const k
   const int64_t blocks = (int64_t)batch * max_new;                   // one CTA per (sequence, new token)
   KB_REQUIRE(blocks < (1ll << 31), "kv_write: too many tokens for one launch");
   cudaStream_t st = (cudaStream_t)stream;
-  if (bf16 && fp8) kv_write_kernel<true, true><<<(unsigned)blocks, kKvWriteThreads, 0, st>>>(p);
-  else if (bf16) kv_write_kernel<true, false><<<(unsigned)blocks, kKvWriteThreads, 0, st>>>(p);
-  else if (fp8) kv_write_kernel<false, true><<<(unsigned)blocks, kKvWriteThreads, 0, st>>>(p);
-  else kv_write_kernel<false, false><<<(unsigned)blocks, kKvWriteThreads, 0, st>>>(p);
+  if (bf16 && fp8) launch_kv_write<true, true>(p, blocks, st);
+  else if (bf16) launch_kv_write<true, false>(p, blocks, st);
+  else if (fp8) launch_kv_write<false, true>(p, blocks, st);
+  else launch_kv_write<false, false>(p, blocks, st);
   KB_CHECK_LAUNCH("kv_write_kernel");
   return 0;
 }

@@ -146,3 +146,29 @@ def test_prefill_to_paged_decode_hand_off():
         got = paged.paged_decode_forward(l, q[:, :, 0], kc, vc, bt, full + 1, D ** -0.5, L + 1)
         assert torch.equal(got, want[:, 0]), f"layer {l}: paged decode differs from the contiguous cache"
     assert nat.read_status() == 0
+
+
+@pytest.mark.parametrize("cache", ["fp16", "bf16", "fp8"])
+@pytest.mark.parametrize("G", [1, 8, 12, 13])
+def test_many_tokens_without_queries_equal_few_at_a_time(cache, G):
+    """Appends of up to 12 KV heads without Q (one step per warp) of more tokens than the SMs hold CTAs run a build of the
+    kernel with fewer registers; the same rows appended 100 at a time do not, and every byte of the caches is the same."""
+    from kascade_b200 import _native as nat
+    dev = torch.device("cuda")
+    g = torch.Generator(device="cuda").manual_seed(G)
+    T, page = 6 * nat.sm_count(0) + 37, 16
+    dtype = torch.bfloat16 if cache == "bf16" else torch.float16
+    k, v = (torch.randn(1, T, G, D, generator=g, device=dev).to(dtype) for _ in range(2))
+    gain = (1 + 0.1 * torch.randn(D, generator=g, device=dev)).to(dtype)
+    pages = -(-(T + 5) // page)
+    table = torch.randperm(pages, generator=g, device=dev).to(torch.int32).view(1, pages)
+    scale = torch.rand(pages, G, generator=g, device=dev) + 0.01 if cache == "fp8" else None
+    filled = []
+    for step in (T, 100):
+        kc, vc = (torch.zeros(pages, page, G, D, dtype=torch.uint8 if cache == "fp8" else dtype, device=dev) for _ in range(2))
+        kv = nat.kv_layout_paged(kc, vc, table, scale, scale)
+        for t in range(0, T, step):
+            at = torch.tensor([5 + t], dtype=torch.int32, device=dev)
+            nat.kv_write(None, None, k[:, t:t + step], v[:, t:t + step], at, None, kv, None, gain, 1e-6, _inv_freq(10000.0).to(dev))
+        filled.append((kc, vc))
+    assert torch.equal(filled[0][0], filled[1][0]) and torch.equal(filled[0][1], filled[1][1])
