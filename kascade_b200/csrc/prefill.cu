@@ -163,11 +163,12 @@ __device__ __forceinline__ float ex2_fma(float x) {
   q = fmaf(q, f, 1.0f);
   return __uint_as_float(__float_as_uint(q) + (__float_as_uint(t) << 23));
 }
-// Which exponentials take that way: of every eight values the fourth and eighth in the lse pass, and the second as
-// well in the pool pass.  The two-element fma occupies the heavy FMA pipe for two cycles, so that pipe (256 + 56 s
-// cycles per block with s of 16 values) and the special-function unit (1024 - 64 s) meet at s = 5-6.  Measured at
-// 8192 tokens, s = 0 / 3 / 4 / 5 / 6 / 16: pool 364 / 313 / 301 / 292 / 295 / 481 us, lse 361 / 325 / 326 / 331 / 333 /
-// 494 us.  The choice is part of the scores' last bits, and so of which of two equal keys is selected.
+// Which exponentials take that way: of every eight values the fourth and eighth in the lse pass (s = 4 of 16), and the
+// second as well in the pool pass (s = 6).  The two-element fma occupies the heavy FMA pipe for two cycles, so that pipe
+// (256 + 56 s cycles per block) and the special-function unit (1024 - 64 s) meet at s = 6.4.  Measured at 8192 tokens,
+// s = 0 / 3 / 4 / 5 / 6 / 16: pool 364 / 313 / 301 / 292 / 295 / 481 us, lse 361 / 325 / 326 / 331 / 333 / 494 us: 5 and 3 were
+// fastest by 1 % and less.  6 and 4 are what the scores were computed with before the two-element forms, and are kept for
+// that: the choice is part of the scores' last bits, and so of which of two nearly equal keys is selected.
 __device__ __forceinline__ float max3(float a, float b, float c) {
   float d;
   asm("max.f32 %0, %1, %2, %3;\n" : "=f"(d) : "f"(a), "f"(b), "f"(c));
