@@ -163,9 +163,9 @@ __host__ __device__ constexpr int dec_warps(int kv) { return kv == 2 ? kDecWarps
 // load that everything else waits for, about a microsecond, so it is done where a CTA has 8192 keys or more (the dense
 // pass of long sequences; see launch_attn).  32 is what one sequence per lane allows, not a measured limit; larger
 // batches are taken as they come.  With 8 KV heads and one split 32 sequences are 256 CTAs, fewer than two per SM, so
-// in practice a batch is ranked where its caller gave the mean length and was given more splits.  Done everywhere, a step of 8 layers of 24 sequences of 4096 to 65536
-// tokens took 1492 us instead of 1563, but 32 of up to 16000 tokens 622 instead of 584, and 5 of up to 50000 353 instead
-// of 334; as it is now 1479, 584 and 334 us.
+// in practice a batch is ranked where its caller gave the mean length and was given more splits.  Done everywhere, a
+// step of 8 layers of 24 sequences of 4096 to 65536 tokens took 1492 us instead of 1563, but 32 of up to 16000 tokens
+// 622 instead of 584, and 5 of up to 50000 353 instead of 334; as it is now 1479, 584 and 334 us.
 constexpr int kRankMax = 32;
 template <typename Len>
 __device__ __forceinline__ int longest_first(int r, int n, const Len& len) {

@@ -700,10 +700,10 @@ static int topk_cluster(int64_t rows, int n_cols) {
 // 3008 x 3001 88 / 50 / 40, 2048 x 8192 92 / 63 / 58, 8192 x 32768 626 / 490 / 505, 24576 x 98304 3776 / 3428 / 7405;
 // decode rows 512 x 32768 68 / 61 / 77, 256 x 16000 23 / 25 / 37, 192 x 65536 58 / 73 / 435.
 // The longer the rows, the more of the time is passes over them and the more the last CTAs to end weigh, above all
-// where the rows differ in length: beyond 32768 scores eight warps need rows for several rounds.  us with 16 / 8:
-// 512 rows of up to 65536 / 131072 scores 96 / 101, 161 / 194; 600 equal ones 154 / 171, 278 / 317; 1024 212 / 208, 389 / 392,
-// of up to that many 156 / 159, 261 / 289; 2048 equal ones 406 / 392, 738 / 745.  A second round of a few rows costs as much: 600 x 24000 / 32768 75.5 / 73.9, 91.2 / 95.5,
-// 800 x 32768 107.4 / 104.4.
+// where the rows differ in length: beyond 32768 scores eight warps need rows for several rounds.  us with 16 / 8: 512
+// rows of up to 65536 / 131072 scores 96 / 101, 161 / 194; 600 equal ones 154 / 171, 278 / 317; 1024 212 / 208, 389 / 392, of up
+// to that many 156 / 159, 261 / 289; 2048 equal ones 406 / 392, 738 / 745.  A second round of a few rows costs as much:
+// 600 x 24000 / 32768 75.5 / 73.9, 91.2 / 95.5, 800 x 32768 107.4 / 104.4.
 static int topk_warps(int64_t rows, int n_cols) {
   const int64_t sms = sm_count();
   if (rows < 3 * sms) return 16;
